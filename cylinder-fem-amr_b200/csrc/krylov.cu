@@ -5,10 +5,15 @@
 // 172-177, :674-679). Here each dot product is fused into the kernel that produces its operand:
 // every block publishes fixed-order partials, the last block to finish sums them in a fixed
 // order and computes the recurrence scalars (alpha, beta, omega, stopping flags) into a state
-// struct in device memory that the following kernels read. A solve is one CUDA graph: the
-// initialisation kernels followed by a conditional WHILE node whose body is one iteration; the
-// body's kernels clear the condition when the solve stops, so the loop runs on the device with
-// no host round trip. Results are deterministic run to run.
+// struct in device memory that the following kernels read. A solve is its initialisation kernels
+// followed by a CUDA graph: a conditional WHILE node whose body is one iteration; the body's
+// kernels clear the condition when the solve stops, so the loop runs on the device with no host
+// round trip. The initialisation is what reads the caller's arrays; the loop works on the
+// context's workspaces, the operator's tiles and the preconditioner's handle, so its graph is
+// captured once per handle and serves any arrays. With the arrays' addresses in the key, three
+// step states in turn on one context re-captured and re-planned at every solve: 15.4 against 12.4
+// ms for one state at 402k vertices, 4.7 against 3.2 ms at 22k, 147 against 135 ms at 4.2M.
+// Results are deterministic run to run.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -508,12 +513,23 @@ k_cg_resid0(int n, const double* __restrict__ b, const double* __restrict__ q, d
     }
 }
 
-__global__ void k_cg_nullx(int n, double* __restrict__ x, double* __restrict__ p0, const CgState* __restrict__ st) {
+// The iteration's own copy of x (zero for b = 0) and p = 0: the loop's graph then holds no
+// address of the caller's, and one graph serves every right-hand side and solution array.
+__global__ void k_cg_start(int n, const double* __restrict__ x0, double* __restrict__ x, double* __restrict__ p0,
+                           const CgState* __restrict__ st) {
     CFA_GRID_DEP();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (st->nullb) x[i] = 0.0;
+    x[i] = st->nullb ? 0.0 : x0[i];
     p0[i] = 0.0;
+}
+
+// First node of a loop's graph: the WHILE condition from the state that the kernels before the
+// graph left.
+template <class S>
+__global__ void k_loop_enter(const S* __restrict__ st, CondArg cond) {
+    CFA_GRID_DEP();
+    if (threadIdx.x == 0 && blockIdx.x == 0) set_cond(cond, st->done ? 0u : 1u);
 }
 
 // 1 / diag (k_extract_inv_diag, src/cfa/linalg.cuh:28-48)
@@ -685,9 +701,9 @@ template <int TPR>
 __global__ void __launch_bounds__(kThreads)
 k_b2_init(int n, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ val,
           const double* __restrict__ xu, const double* __restrict__ xv, const double* __restrict__ bu,
-          const double* __restrict__ bv, double2* __restrict__ r, double2* __restrict__ r0, double2* __restrict__ p,
-          double2* __restrict__ vv, B2State* __restrict__ st, double* __restrict__ part, unsigned int* __restrict__ counter,
-          CondArg cond) {
+          const double* __restrict__ bv, double2* __restrict__ x, double2* __restrict__ r, double2* __restrict__ r0,
+          double2* __restrict__ p, double2* __restrict__ vv, B2State* __restrict__ st, double* __restrict__ part,
+          unsigned int* __restrict__ counter, CondArg cond) {
     CFA_GRID_DEP();
     __shared__ double sh[2 * kWarps];
     double acc[2] = {0.0, 0.0};
@@ -705,6 +721,7 @@ k_b2_init(int n, const int* __restrict__ rp, const int* __restrict__ ci, const d
     if (valid && lane == 0) {
         const double ru = bu[row] - 1.0 * su, rv = bv[row] - 1.0 * sv;
         const double2 rr = make_double2(ru, rv);
+        x[row] = make_double2(xu[row], xv[row]);
         r[row] = rr;
         r0[row] = rr;
         p[row] = rr;
@@ -871,8 +888,8 @@ k_b2_t(int n, const int* __restrict__ rp, const int* __restrict__ ci, const doub
 // x += a1 phat + a2 shat, r = s - cw t; r.r, r0.r -> stop tests, rho (:737-750); then the
 // start of the next iteration
 __global__ void __launch_bounds__(kThreads)
-k_b2_xr(int n, double* __restrict__ xu, double* __restrict__ xv, const double2* __restrict__ phat,
-        const double2* __restrict__ shat, const double2* __restrict__ s, const double2* __restrict__ t,
+k_b2_xr(int n, double2* __restrict__ x, const double2* __restrict__ phat, const double2* __restrict__ shat,
+        const double2* __restrict__ s, const double2* __restrict__ t,
         double2* __restrict__ r, const double2* __restrict__ r0, B2State* __restrict__ st, double* __restrict__ part,
         unsigned int* __restrict__ counter, CondArg cond) {
     CFA_GRID_DEP();
@@ -882,8 +899,10 @@ k_b2_xr(int n, double* __restrict__ xu, double* __restrict__ xv, const double2* 
     double acc[4] = {0, 0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const double2 ph = phat[i], sh2 = shat[i], ss = s[i], tt = t[i], q = r0[i];
-        xu[i] += a10 * ph.x + a20 * sh2.x;
-        xv[i] += a11 * ph.y + a21 * sh2.y;
+        double2 xx = x[i];
+        xx.x += a10 * ph.x + a20 * sh2.x;
+        xx.y += a11 * ph.y + a21 * sh2.y;
+        x[i] = xx;
         const double ru = ss.x - w0 * tt.x, rv = ss.y - w1 * tt.y;
         r[i] = make_double2(ru, rv);
         acc[0] += ru * ru; acc[1] += rv * rv;
@@ -916,16 +935,27 @@ k_b2_xr(int n, double* __restrict__ xu, double* __restrict__ xv, const double2* 
     }
 }
 
+// The solution pair to the caller's two arrays
+__global__ void k_b2_out(int n, const double2* __restrict__ x, double* __restrict__ xu, double* __restrict__ xv) {
+    CFA_GRID_DEP();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double2 v = x[i];
+        xu[i] = v.x;
+        xv[i] = v.y;
+    }
+}
+
 // ---- tile-streamed forms of the BiCGSTAB2 SpMV + dot kernels (tiles of {A}, FP64) ----
-// MODE 0: init  (x -> v = A x, r = b - v, r0 = p = r, v = 0, r.r)
+// MODE 0: init  (x -> v = A x, r = b - v, r0 = p = r, v = 0, the pair x, r.r)
 // MODE 1: v = A phat, r0.v -> alpha
 // MODE 2: t = A shat, s.s t.t t.s -> omega / s-stop
 template <int TPR, int MODE>
 __global__ void __launch_bounds__(kTileThreads)
 k_b2t(TileView tv, int n, const double* __restrict__ xu, const double* __restrict__ xv, const double* __restrict__ bu,
       const double* __restrict__ bv, const double2* __restrict__ in, const double2* __restrict__ aux,
-      double2* __restrict__ out, double2* __restrict__ r, double2* __restrict__ r0, double2* __restrict__ p,
-      B2State* __restrict__ st, double* __restrict__ part, unsigned int* __restrict__ counter, CondArg cond) {
+      double2* __restrict__ out, double2* __restrict__ x, double2* __restrict__ r, double2* __restrict__ r0,
+      double2* __restrict__ p, B2State* __restrict__ st, double* __restrict__ part,
+      unsigned int* __restrict__ counter, CondArg cond) {
     extern __shared__ __align__(128) unsigned char tsmem[];
     constexpr int NV = MODE == 2 ? 6 : 2;
     __shared__ double sh[NV * kWarps];
@@ -979,6 +1009,7 @@ k_b2t(TileView tv, int n, const double* __restrict__ xu, const double* __restric
                 if (MODE == 0) {
                     const double ru = bu[row] - 1.0 * su, rv = bv[row] - 1.0 * sv;
                     const double2 rr = make_double2(ru, rv);
+                    x[row] = make_double2(xu[row], xv[row]);
                     r[row] = rr;
                     r0[row] = rr;
                     p[row] = rr;
@@ -1117,6 +1148,30 @@ struct GraphCache {
     ~GraphCache() { reset(); }
 };
 
+// The loop graphs a context keeps, by key (the handle that the loop applies, the plan, the
+// workspaces): a program that alternates a few hierarchies or factors, as one with several meshes
+// does, captures each loop once. The least recently used one makes room.
+struct GraphSet {
+    static constexpr int kSlots = 4;
+    GraphCache g[kSlots];
+    unsigned long long stamp[kSlots] = {0, 0, 0, 0}, clock = 0;
+    GraphCache& slot(const std::vector<const void*>& key) {
+        int best = 0;
+        for (int k = 0; k < kSlots; ++k) {
+            if (g[k].exec && g[k].key == key) { best = k; break; }
+            if (stamp[k] < stamp[best]) best = k;
+        }
+        stamp[best] = ++clock;
+        return g[best];
+    }
+    void reset() {
+        for (int k = 0; k < kSlots; ++k) {
+            g[k].reset();
+            stamp[k] = 0;
+        }
+    }
+};
+
 // A straight-line captured graph (no conditional node), replayed while its key holds
 struct SegGraph {
     cudaGraphExec_t exec = nullptr;
@@ -1132,7 +1187,7 @@ struct SegGraph {
 
 struct PcgWork {
     int cap = 0;
-    DevBuf<double> r, z, p, pn, q, gx, gy, dinv;
+    DevBuf<double> x, r, z, p, pn, q, gx, gy, dinv;
     DevBuf<double> c0;                 // omega0 D0^-1 r for the V-cycle's level 0 (float or double elements)
     DevBuf<CgState> st;
     // tile-streamed copy of the operator: K - B^T M^-1 B as one matrix on the two-ring pattern
@@ -1148,23 +1203,25 @@ struct PcgWork {
     DevBuf<int> err;
     DevBuf<double> part;
     DevBuf<unsigned int> counter;
-    GraphCache graph;
-    GraphCache graph2;   // the second phase of a mixed-precision solve (FP32 V-cycles)
+    GraphSet graph;
+    GraphSet graph2;   // the second phase of a mixed-precision solve (FP32 V-cycles)
     SegGraph seg[3];   // the pieces of one iteration between host hooks (cfa_pcg_solve_host_ops)
     DevBuf<unsigned long long> fp;
 };
 
 struct B2Work {
     int cap = 0;
-    DevBuf<double> r, r0, p, v, s, t, phat, shat;
+    DevBuf<double> x, r, r0, p, v, s, t, phat, shat;
     DevBuf<B2State> st;
     TiledCsr tA;                     // tile-streamed copy of the momentum matrix (packed per solve)
     std::vector<const void*> tile_key;
+    unsigned long long tile_fp = 0;  // fingerprint of the planned pattern
+    DevBuf<unsigned long long> fp;
     bool tiled = false;
     DevBuf<int> err;
     DevBuf<double> part;
     DevBuf<unsigned int> counter;
-    GraphCache graph;
+    GraphSet graph;
 };
 
 struct SolverWork {
@@ -1185,6 +1242,18 @@ void free_solver_work(cfa_ctx* ctx) {
 static bool graphs_enabled() {
     const char* e = std::getenv("CFA_GRAPHS");
     return !(e && e[0] == '0');
+}
+
+// The environment switches that choose kernels while a loop is captured, as one word of its key.
+static const void* loop_switches() {
+    unsigned long long h = 1469598103934665603ull;   // FNV-1a over the values
+    for (const char* name : {"CFA_ILU_PERM", "CFA_ILU_STAGED", "CFA_PRESCALE", "CFA_CG_FUSE_UPDATE",
+                             "CFA_PCG_FLEXIBLE", "CFA_VCYCLE_FP64", "CFA_L2_OP", "CFA_L2_VC"}) {
+        const char* e = std::getenv(name);
+        for (const char* c = e ? e : "-"; *c; ++c) h = (h ^ (unsigned char)*c) * 1099511628211ull;
+        h = (h ^ 0xffu) * 1099511628211ull;
+    }
+    return (const void*)(uintptr_t)h;
 }
 
 // Captures `init` then a WHILE node with `body` into `gc` (the init kernels set the condition).
@@ -1235,6 +1304,13 @@ static cfa_status build_graph(cfa_ctx* ctx, GraphCache& gc, Init init, Body body
     if (s != CFA_OK) return s;
     CFA_CUDA(e);
     CFA_CUDA(cudaGraphInstantiate(&gc.exec, g, 0));
+    return CFA_OK;
+}
+
+template <class S>
+static cfa_status loop_enter(cfa_ctx* ctx, const S* st, CondArg cond) {
+    CFA_LAUNCH(ctx, k_loop_enter<S>, 1, 32, 0, st, cond);
+    CFA_CHECK_LAUNCH();
     return CFA_OK;
 }
 
@@ -1410,7 +1486,7 @@ static cfa_status pcg_init(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, CondArg c
     } else {
         CFA_LAUNCH(ctx, k_vmul, gv, kThreads, 0, n, W.dinv.p, W.r.p, W.z.p);
     }
-    CFA_LAUNCH(ctx, k_cg_nullx, ceil_div(n, kThreads), kThreads, 0, n, a.x, W.p.p, st);
+    CFA_LAUNCH(ctx, k_cg_start, ceil_div(n, kThreads), kThreads, 0, n, (const double*)a.x, W.x.p, W.p.p, st);
     CFA_LAUNCH(ctx, k_cg_rz, gv, kThreads, 0, n, W.r.p, W.z.p, (const double*)W.q.p, 1, 0, st, W.part.p,
                W.counter.p, cond);
     CFA_CHECK_LAUNCH();
@@ -1451,15 +1527,15 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
             const bool prescale = !a.prec && !fuse_update && amg_prescale(a.amg, &ps, a.vc64 != 0);
             if (!fuse_update) {
                 if (prescale && ps.fp32)
-                    CFA_LAUNCH(ctx, (k_cg_update<false, float>), gv, kThreads, 0, n, a.x, W.r.p, W.pn.p, W.p.p, W.q.p,
+                    CFA_LAUNCH(ctx, (k_cg_update<false, float>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p, W.q.p,
                                (const double*)nullptr, (double*)nullptr, st, W.part.p, W.counter.p, cond,
                                (const float*)ps.dinv, (float)ps.omega, reinterpret_cast<float*>(W.c0.p));
                 else if (prescale)
-                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, a.x, W.r.p, W.pn.p, W.p.p,
+                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p,
                                W.q.p, (const double*)nullptr, (double*)nullptr, st, W.part.p, W.counter.p, cond,
                                (const double*)ps.dinv, ps.omega, W.c0.p);
                 else
-                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, a.x, W.r.p, W.pn.p, W.p.p,
+                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p,
                                W.q.p, (const double*)nullptr, (double*)nullptr, st, W.part.p, W.counter.p, cond,
                                (const double*)nullptr, 0.0, (double*)nullptr);
             }
@@ -1467,7 +1543,7 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
                 // z = M^-1 r with r.z (and z.q) folded into the V-cycle's last sweep where it can be
                 const int flexible = pcg_flexible(a.amg);
                 const RzFuse f{W.q.p, flexible, &st->rz, &st->beta, &st->alpha, W.part.p, W.counter.p};
-                const CgFuse g{W.r.p, W.q.p, W.pn.p, a.x, W.p.p, st, W.part.p, W.counter.p, cond};
+                const CgFuse g{W.r.p, W.q.p, W.pn.p, W.x.p, W.p.p, st, W.part.p, W.counter.p, cond};
                 bool fused = false;
                 CFA_PROPAGATE(amg_vcycle_rz(ctx, a.amg, W.r.p, W.z.p, done, f, &fused, fuse_update ? &g : nullptr,
                                             prescale ? (const void*)W.c0.p : nullptr, a.vc64 != 0));
@@ -1476,7 +1552,7 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
                                W.part.p, W.counter.p, cond);
             }
         } else {
-            CFA_LAUNCH(ctx, (k_cg_update<true, double>), gv, kThreads, 0, n, a.x, W.r.p, W.pn.p, W.p.p, W.q.p, W.dinv.p, W.z.p,
+            CFA_LAUNCH(ctx, (k_cg_update<true, double>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p, W.q.p, W.dinv.p, W.z.p,
                        st, W.part.p, W.counter.p, cond, (const double*)nullptr, 0.0, (double*)nullptr);
         }
     } else if (a.prec) {
@@ -1587,7 +1663,7 @@ static cfa_status ensure_pcg_vectors(cfa_ctx* ctx, PcgWork& W, int n) {
         W.graph.reset();
         W.graph2.reset();
         for (SegGraph& g : W.seg) g.reset();
-        for (DevBuf<double>* b : {&W.r, &W.z, &W.p, &W.pn, &W.q, &W.gx, &W.gy, &W.dinv, &W.c0}) CFA_CUDA(b->ensure(n));
+        for (DevBuf<double>* b : {&W.x, &W.r, &W.z, &W.p, &W.pn, &W.q, &W.gx, &W.gy, &W.dinv, &W.c0}) CFA_CUDA(b->ensure(n));
         CFA_CUDA(W.st.ensure(1));
         CFA_CUDA(W.counter.ensure(1));
         CFA_CUDA(cudaMemsetAsync(W.counter.p, 0, sizeof(unsigned int), ctx->stream));
@@ -1682,9 +1758,11 @@ static cfa_status plan_operator_tiles(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a
     W.tiled = tiles_enabled();
     if (!W.tiled) return CFA_OK;
     allow_operator_kernels();
-    std::vector<const void*> key = {a.rp, a.ci, (const void*)(intptr_t)a.n, (const void*)(intptr_t)a.nnz,
+    // the pattern's content alone: another copy of it at other addresses keeps the plan
+    std::vector<const void*> key = {(const void*)(intptr_t)a.n, (const void*)(intptr_t)a.nnz,
                                     (const void*)(intptr_t)(a.oss ? 1 : 0), (const void*)(uintptr_t)a.fp};
     if (key == W.tile_key) return CFA_OK;
+    W.tile_key.clear();
     std::vector<int> h_rp(a.n + 1);
     CFA_CUDA(cudaMemcpyAsync(h_rp.data(), a.rp, (a.n + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CFA_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1716,13 +1794,13 @@ static cfa_status plan_operator_tiles(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a
 }
 
 // nnz = rp[n] and the pattern's fingerprint, one synchronisation
-static cfa_status pattern_info(cfa_ctx* ctx, int n, const int* rp, const int* ci, int& nnz, unsigned long long& fp) {
-    PcgWork& W = work(ctx)->pcg;
-    CFA_CUDA(W.fp.ensure(1));
-    CFA_CUDA(cudaMemsetAsync(W.fp.p, 0, sizeof(unsigned long long), ctx->stream));
+static cfa_status pattern_info(cfa_ctx* ctx, DevBuf<unsigned long long>& d_fp, int n, const int* rp, const int* ci,
+                               int& nnz, unsigned long long& fp) {
+    CFA_CUDA(d_fp.ensure(1));
+    CFA_CUDA(cudaMemsetAsync(d_fp.p, 0, sizeof(unsigned long long), ctx->stream));
     CFA_LAUNCH(ctx, k_pattern_fingerprint, std::min(ceil_div(8 * n + 1, kThreads), 4 * ctx->num_sms), kThreads, 0, n, rp,
-               ci, W.fp.p);
-    CFA_CUDA(cudaMemcpyAsync(&ctx->h_pinned[0], W.fp.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+               ci, d_fp.p);
+    CFA_CUDA(cudaMemcpyAsync(&ctx->h_pinned[0], d_fp.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                              ctx->stream));
     CFA_CUDA(cudaMemcpyAsync(&ctx->h_pinned[1], rp + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CFA_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1749,38 +1827,50 @@ static cfa_status pcg_solve(cfa_ctx* ctx, const PcgArgs& a, cfa_solve_report* re
     CFA_CUDA(cudaMemcpyAsync(W.st.p, &init, sizeof(CgState), cudaMemcpyHostToDevice, ctx->stream));
     CFA_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     long long extra_body = 0;
+    // Loop graphs: with the operator in its tiles the body touches the workspaces, the plan and the
+    // hierarchy only, so those are its key; the forms that read the caller's arrays in every
+    // iteration (two-pass OSS, no tiles) key on their addresses too.
     const cfa_mesh* om = a.oss ? a.oss->mesh : nullptr;
-    const std::vector<const void*> key = {a.rp, a.ci, a.val, a.b, a.x, a.oss ? a.oss->d_oss_val : nullptr,
-                                          a.oss ? a.oss->d_inv_m : nullptr, (const void*)(intptr_t)(om ? om->uid : 0),
-                                          (const void*)(intptr_t)(om ? om->bc.outlet_dirichlet : 0),
-                                          (const void*)(intptr_t)(om ? om->bc.pin : 0),
-                                          (const void*)(intptr_t)(a.amg ? a.amg->version : 0),
-                                          (const void*)(intptr_t)n, (const void*)(intptr_t)a.nnz,
-                                          (const void*)(intptr_t)((a.extra ? 1 : 0) | (a.prec ? 2 : 0)),
-                                          (const void*)(uintptr_t)a.fp};
+    std::vector<const void*> key = {(const void*)(intptr_t)(a.amg ? a.amg->version : 0), (const void*)(intptr_t)n,
+                                    (const void*)(intptr_t)a.nnz,
+                                    (const void*)(intptr_t)((a.extra ? 1 : 0) | (a.prec ? 2 : 0) | (a.oss ? 4 : 0) |
+                                                            (W.tiled ? 8 : 0) | (two ? 16 : 0)),
+                                    (const void*)(uintptr_t)a.fp, loop_switches()};
+    if (!W.tiled || (a.oss && !W.fused)) {
+        const void* more[] = {a.rp, a.ci, a.val, a.oss ? a.oss->d_oss_val : nullptr, a.oss ? a.oss->d_inv_m : nullptr,
+                              (const void*)(intptr_t)(om ? om->uid : 0),
+                              (const void*)(intptr_t)(om ? om->bc.outlet_dirichlet : 0),
+                              (const void*)(intptr_t)(om ? om->bc.pin : 0)};
+        key.insert(key.end(), std::begin(more), std::end(more));
+    }
+    CondArg none{0, 0};
+    CFA_PROPAGATE(pcg_init(ctx, W, a1, none));
     if (graphs_enabled() && !a.host_ops()) {
-        std::vector<const void*> key1 = key;
-        key1.push_back((const void*)(intptr_t)(two ? 1 : 0));
-        if (!W.graph.exec || W.graph.key != key1) {
-            CFA_PROPAGATE(build_graph(ctx, W.graph, [&](CondArg c) { return pcg_init(ctx, W, a1, c); },
+        GraphCache& g1 = W.graph.slot(key);
+        if (!g1.exec || g1.key != key) {
+            CFA_PROPAGATE(build_graph(ctx, g1, [&](CondArg c) { return loop_enter(ctx, W.st.p, c); },
                                       [&](CondArg c) { return pcg_body(ctx, W, a1, c); }));
-            W.graph.key = key1;
+            g1.key = key;
         }
-        CFA_CUDA(cudaGraphLaunch(W.graph.exec, ctx->stream));
-        extra_body = W.graph.body_kernels;
-        ctx->launches += W.graph.init_kernels;
+        CFA_CUDA(cudaGraphLaunch(g1.exec, ctx->stream));
+        extra_body = g1.body_kernels;
+        ctx->launches += g1.init_kernels;
         if (two) {
-            if (!W.graph2.exec || W.graph2.key != key) {
-                CFA_PROPAGATE(build_graph(ctx, W.graph2, [&](CondArg c) { return pcg_resume(ctx, W, a, a.tol, c); },
+            // the switch and final tolerances are data of the second graph's first kernel
+            std::vector<const void*> key2 = key;
+            unsigned long long tol_bits;
+            std::memcpy(&tol_bits, &a.tol, sizeof(tol_bits));
+            key2.push_back((const void*)(uintptr_t)tol_bits);
+            GraphCache& g2 = W.graph2.slot(key2);
+            if (!g2.exec || g2.key != key2) {
+                CFA_PROPAGATE(build_graph(ctx, g2, [&](CondArg c) { return pcg_resume(ctx, W, a, a.tol, c); },
                                           [&](CondArg c) { return pcg_body(ctx, W, a, c); }));
-                W.graph2.key = key;
+                g2.key = key2;
             }
-            CFA_CUDA(cudaGraphLaunch(W.graph2.exec, ctx->stream));
-            ctx->launches += W.graph2.init_kernels;
+            CFA_CUDA(cudaGraphLaunch(g2.exec, ctx->stream));
+            ctx->launches += g2.init_kernels;
         }
     } else {
-        CondArg none{0, 0};
-        CFA_PROPAGATE(pcg_init(ctx, W, a1, none));
         const bool segments = graphs_enabled();   // host hooks: one graph per piece of the iteration
         for (int phase = 0; phase < (two ? 2 : 1); ++phase) {
             const PcgArgs& ap = phase == 0 ? a1 : a;
@@ -1799,6 +1889,7 @@ static cfa_status pcg_solve(cfa_ctx* ctx, const PcgArgs& a, cfa_solve_report* re
             }
         }
     }
+    CFA_CUDA(cudaMemcpyAsync(a.x, W.x.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     CFA_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     CgState h;
     int h_err = 0;
@@ -1855,8 +1946,8 @@ static void launch_b2t(cfa_ctx* ctx, B2Work& W, const B2Args& a, const double* i
     TILE_TPR_SWITCH(W.tA.tpr,
         L = tile_launch(ctx, W.tA, (const void*)k_b2t<TPR, MODE>);
         CFA_LAUNCH(ctx, (k_b2t<TPR, MODE>), L.grid, kTileThreads, L.smem, tv, a.n, (const double*)a.xu,
-                   (const double*)a.xv, a.bu, a.bv, pair(in), pair(aux), pair(out), pair(W.r.p), pair(W.r0.p),
-                   pair(W.p.p), W.st.p, W.part.p, W.counter.p, cond));
+                   (const double*)a.xv, a.bu, a.bv, pair(in), pair(aux), pair(out), pair(W.x.p), pair(W.r.p),
+                   pair(W.r0.p), pair(W.p.p), W.st.p, W.part.p, W.counter.p, cond));
 }
 
 template <int TPR>
@@ -1883,11 +1974,21 @@ static cfa_status plan_b2_tiles(cfa_ctx* ctx, B2Work& W, const B2Args& a) {
     std::vector<const void*> key = {a.rp, a.ci, (const void*)(intptr_t)a.n, (const void*)(intptr_t)a.nnz,
                                     (const void*)(intptr_t)a.ilu->uid};
     if (key == W.tile_key) return CFA_OK;
+    // another handle or other arrays: the plan is kept when the pattern's content is the planned one
+    int nnz = 0;
+    unsigned long long fp = 0;
+    CFA_PROPAGATE(pattern_info(ctx, W.fp, a.n, a.rp, a.ci, nnz, fp));
+    if (W.tA.rows == a.n && W.tA.nnz == nnz && W.tile_fp == fp && !W.tile_key.empty()) {
+        W.tile_key = key;
+        return CFA_OK;
+    }
+    W.tile_key.clear();
     std::vector<int> h_rp(a.n + 1);
     CFA_CUDA(cudaMemcpyAsync(h_rp.data(), a.rp, (a.n + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CFA_CUDA(cudaStreamSynchronize(ctx->stream));
     CFA_PROPAGATE(plan_tiled(ctx, h_rp.data(), a.n, 1, 8, W.tA));
     W.tile_key = key;
+    W.tile_fp = fp;
     W.graph.reset();
     return CFA_OK;
 }
@@ -1902,7 +2003,7 @@ static cfa_status b2_init(cfa_ctx* ctx, B2Work& W, const B2Args& a, CondArg cond
     const int tpr = op_tpr(a.n, a.nnz);
     const int grid = row_grid(ctx, a.n, tpr);
     OP_TPR_SWITCH(tpr, CFA_LAUNCH(ctx, (k_b2_init<TPR>), grid, kThreads, 0, a.n, a.rp, a.ci, a.val, (const double*)a.xu,
-                                  (const double*)a.xv, a.bu, a.bv, pair(W.r.p), pair(W.r0.p), pair(W.p.p),
+                                  (const double*)a.xv, a.bu, a.bv, pair(W.x.p), pair(W.r.p), pair(W.r0.p), pair(W.p.p),
                                   pair(W.v.p), W.st.p, W.part.p, W.counter.p, cond));
     CFA_CHECK_LAUNCH();
     return CFA_OK;
@@ -1932,8 +2033,8 @@ static cfa_status b2_body(cfa_ctx* ctx, B2Work& W, const B2Args& a, CondArg cond
     else
         OP_TPR_SWITCH(tpr, CFA_LAUNCH(ctx, (k_b2_t<TPR>), grid, kThreads, 0, n, a.rp, a.ci, a.val, pair(W.shat.p),
                                       pair(W.s.p), pair(W.t.p), W.st.p, W.part.p, W.counter.p));
-    CFA_LAUNCH(ctx, k_b2_xr, gv, kThreads, 0, n, a.xu, a.xv, pair(W.phat.p), pair(W.shat.p),
-               pair(W.s.p), pair(W.t.p), pair(W.r.p), pair(W.r0.p), W.st.p, W.part.p, W.counter.p, cond);
+    CFA_LAUNCH(ctx, k_b2_xr, gv, kThreads, 0, n, pair(W.x.p), pair(W.phat.p), pair(W.shat.p), pair(W.s.p),
+               pair(W.t.p), pair(W.r.p), pair(W.r0.p), W.st.p, W.part.p, W.counter.p, cond);
     CFA_CHECK_LAUNCH();
     return CFA_OK;
 }
@@ -1943,7 +2044,7 @@ static cfa_status b2_solve(cfa_ctx* ctx, const B2Args& a, cfa_solve_report* rep)
     const int n = a.n;
     if (n > W.cap) {
         W.graph.reset();
-        for (DevBuf<double>* b : {&W.r, &W.r0, &W.p, &W.v, &W.s, &W.t, &W.phat, &W.shat}) CFA_CUDA(b->ensure(2 * (size_t)n));
+        for (DevBuf<double>* b : {&W.x, &W.r, &W.r0, &W.p, &W.v, &W.s, &W.t, &W.phat, &W.shat}) CFA_CUDA(b->ensure(2 * (size_t)n));
         CFA_CUDA(W.st.ensure(1));
         CFA_CUDA(W.counter.ensure(1));
         CFA_CUDA(cudaMemsetAsync(W.counter.p, 0, sizeof(unsigned int), ctx->stream));
@@ -1957,20 +2058,24 @@ static cfa_status b2_solve(cfa_ctx* ctx, const B2Args& a, cfa_solve_report* rep)
     CFA_CUDA(cudaMemcpyAsync(W.st.p, &init, sizeof(B2State), cudaMemcpyHostToDevice, ctx->stream));
     CFA_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     long long extra_body = 0;
+    CondArg none{0, 0};
+    CFA_PROPAGATE(b2_init(ctx, W, a, none));
     if (graphs_enabled()) {
-        std::vector<const void*> key = {a.rp, a.ci, a.val, a.bu, a.bv, a.xu, a.xv, (const void*)(intptr_t)a.ilu->uid,
-                                        (const void*)(intptr_t)n, (const void*)(intptr_t)a.nnz};
-        if (!W.graph.exec || W.graph.key != key) {
-            CFA_PROPAGATE(build_graph(ctx, W.graph, [&](CondArg c) { return b2_init(ctx, W, a, c); },
+        // as in pcg_solve: the loop over the tiles holds no address of the caller's
+        std::vector<const void*> key = {(const void*)(intptr_t)a.ilu->uid, (const void*)(intptr_t)n,
+                                        (const void*)(intptr_t)a.nnz, (const void*)(intptr_t)(W.tiled ? 1 : 0),
+                                        loop_switches()};
+        if (!W.tiled) key.insert(key.end(), {a.rp, a.ci, a.val});
+        GraphCache& g = W.graph.slot(key);
+        if (!g.exec || g.key != key) {
+            CFA_PROPAGATE(build_graph(ctx, g, [&](CondArg c) { return loop_enter(ctx, W.st.p, c); },
                                       [&](CondArg c) { return b2_body(ctx, W, a, c); }));
-            W.graph.key = key;
+            g.key = key;
         }
-        CFA_CUDA(cudaGraphLaunch(W.graph.exec, ctx->stream));
-        extra_body = W.graph.body_kernels;
-        ctx->launches += W.graph.init_kernels;
+        CFA_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
+        extra_body = g.body_kernels;
+        ctx->launches += g.init_kernels;
     } else {
-        CondArg none{0, 0};
-        CFA_PROPAGATE(b2_init(ctx, W, a, none));
         int polled = 0;
         for (int it = 0; it < a.max_iter; ++it) {
             CFA_PROPAGATE(b2_body(ctx, W, a, none));
@@ -1983,6 +2088,7 @@ static cfa_status b2_solve(cfa_ctx* ctx, const B2Args& a, cfa_solve_report* rep)
             }
         }
     }
+    CFA_LAUNCH(ctx, k_b2_out, row_grid(ctx, n, 1), kThreads, 0, n, (const double2*)pair(W.x.p), a.xu, a.xv);
     CFA_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     B2State h;
     int h_err = 0;
@@ -2041,7 +2147,7 @@ cfa_status cfa_pressure_operator_prepare(cfa_ctx* ctx, int n, int nnz, const int
     CFA_PROPAGATE(ensure_pcg_vectors(ctx, W, n));
     int nnz_dev = 0;
     unsigned long long fp = 0;
-    CFA_PROPAGATE(pattern_info(ctx, n, rp, ci, nnz_dev, fp));
+    CFA_PROPAGATE(pattern_info(ctx, W.fp, n, rp, ci, nnz_dev, fp));
     CFA_ARG(nnz_dev == nnz);
     PcgArgs a{n, nnz, rp, ci, val, nullptr, nullptr, oss, nullptr, 0, 0.0};
     a.fp = fp;
@@ -2111,7 +2217,7 @@ cfa_status cfa_pcg_solve(cfa_ctx* ctx, int n, const int* rp, const int* ci, cons
     CFA_ARG(!amg || (amg->coarse_n > 0 && (amg->levels.empty() ? amg->coarse_n == n : amg->levels[0].A.rows == n)));
     int nnz = 0;
     unsigned long long fp = 0;
-    CFA_PROPAGATE(pattern_info(ctx, n, rp, ci, nnz, fp));
+    CFA_PROPAGATE(pattern_info(ctx, work(ctx)->pcg.fp, n, rp, ci, nnz, fp));
     PcgArgs a{n, nnz, rp, ci, val, b, x, oss, amg, opts->max_iter, opts->tol};
     a.fp = fp;
     if (opts->max_iter == 0) {
@@ -2130,7 +2236,7 @@ cfa_status cfa_pcg_solve_host_ops(cfa_ctx* ctx, int n, const int* rp, const int*
     CFA_ARG(!amg || (amg->coarse_n > 0 && (amg->levels.empty() ? amg->coarse_n == n : amg->levels[0].A.rows == n)));
     int nnz = 0;
     unsigned long long fp = 0;
-    CFA_PROPAGATE(pattern_info(ctx, n, rp, ci, nnz, fp));
+    CFA_PROPAGATE(pattern_info(ctx, work(ctx)->pcg.fp, n, rp, ci, nnz, fp));
     PcgArgs a{n, nnz, rp, ci, val, b, x, nullptr, amg, opts->max_iter, opts->tol};
     a.fp = fp;
     a.extra = extra_op;
