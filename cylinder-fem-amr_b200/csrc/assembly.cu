@@ -1,6 +1,9 @@
-// Atomic-free element assembly (a3-a9): one thread per matrix row gathers the contributions of
-// the row's elements from the sorted node -> element incidence, in ascending element order, and
-// writes every value once. Compared with the reference's one-thread-per-element kernels with FP64
+// Atomic-free element assembly (a3-a9). A block owns a tile of consecutive rows and computes each
+// element that touches them once, into shared memory (elemtile.cuh); its threads then sum every
+// CSR entry and right-hand side entry from there, in ascending element order, and write every value
+// once, entries coalesced. Where a tile's elements do not fit (a node of very many elements), one
+// thread per matrix row gathers the contributions of the row's elements from the sorted
+// node -> element incidence, in the same order. Compared with the reference's one-thread-per-element kernels with FP64
 // atomicAdd into a binary-searched CSR slot (src/cfa/fem_kernels.cuh:40-282, :697-909), there
 // are no atomics and no searches, the result is deterministic, and each CSR value is written
 // exactly once (coalesced along the row).
@@ -152,6 +155,114 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
         for (int q = 0; q < len; ++q) A_val[r0 + q] = acc[q * T];
     rhs_u[i] = f_u_row;
     rhs_v[i] = f_v_row;
+}
+
+// Momentum rows on element tiles: the element matrix and right-hand side of every element of the
+// tile (16 doubles an element: A_ab, f_u, f_v, area / 3), then the entries, the rows and the
+// Dirichlet rows. Bound by latency: each block's chain of plan, vertices and fields, the divisions
+// and square roots of the element formula, then the entries' codes. Against the row gather: 142 ->
+// 130 us at 402k vertices (130 MB, 1.0 TB/s), 21.0 -> 13.3 us at 22.5k, 19.5 -> 13.2 us at 8k.
+__global__ void __launch_bounds__(kEtThreads)
+k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
+                 const double* __restrict__ y, const int* __restrict__ tag, const int* __restrict__ rp,
+                 const int* __restrict__ ci, const double* __restrict__ u_old, const double* __restrict__ v_old,
+                 const double* __restrict__ u_prev, const double* __restrict__ v_prev,
+                 const double* __restrict__ p_old, const double* __restrict__ nu_node, MomParams P, int with_bc,
+                 double u_max, double H, OutletBc bc, double* __restrict__ A_val, double* __restrict__ rhs_u,
+                 double* __restrict__ rhs_v, double* __restrict__ mass) {
+    extern __shared__ __align__(16) double et_rec[];   // [16][tv.stride]
+    const EtBlock b = et_block(tv, n);
+    const int S = tv.stride;
+    CFA_GRID_DEP();
+    constexpr double kThird = 1.0 / 3.0, kSixth = 1.0 / 6.0, kTwelfth = 1.0 / 12.0;
+    const double inv_rho = 1.0 / P.rho, term_t = 2.0 / P.tau_time;
+    for (int le = threadIdx.x; le < b.ne; le += kEtThreads) {
+        int nd[3];
+        load_elem(ev, tv.elems[b.i0 + le], nd);
+        const Geom g = elem_geom(nd, x, y);
+        double* rec = et_rec + le;
+        if (!g.ok) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) rec[q * S] = 0.0;
+            continue;
+        }
+        const double area = g.area, area3 = area * kThird;
+        double u_h[3], v_h[3], w_u = 0.0, w_v = 0.0, div_w = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double un = u_old[nd[k]], vn = v_old[nd[k]], um = u_prev[nd[k]], vm = v_prev[nd[k]];
+            u_h[k] = P.a1 * un + P.a2 * um;
+            v_h[k] = P.a1 * vn + P.a2 * vm;
+            const double wu = P.c1 * un + P.c2 * um, wv = P.c1 * vn + P.c2 * vm;
+            w_u += wu * kThird;
+            w_v += wv * kThird;
+            div_w += wu * g.dNdx[k] + wv * g.dNdy[k];
+        }
+        const double vel_mag = sqrt(w_u * w_u + w_v * w_v) + 1.0e-12;
+        const double h_K = sqrt(2.0 * area);
+        // element viscosity: the scalar nu, or the mean of a nodal field
+        const double nu = nu_node ? (nu_node[nd[0]] + nu_node[nd[1]] + nu_node[nd[2]]) * kThird : P.nu;
+        const double term_c = 2.0 * vel_mag / h_K;
+        const double term_d = 4.0 * nu / (h_K * h_K);
+        const double tau_supg = 1.0 / sqrt(term_t * term_t + term_c * term_c + 9.0 * term_d * term_d);
+        const double p0 = p_old[nd[0]], p1 = p_old[nd[1]], p2 = p_old[nd[2]];
+        const double dpdx = (p0 * g.dNdx[0] + p1 * g.dNdx[1] + p2 * g.dNdx[2]) * inv_rho;
+        const double dpdy = (p0 * g.dNdy[0] + p1 * g.dNdy[1] + p2 * g.dNdy[2]) * inv_rho;
+        double ugN[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ugN[k] = w_u * g.dNdx[k] + w_v * g.dNdy[k];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            double f_u = 0.0, f_v = 0.0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const double M_ij = (a == j) ? (area * kSixth) : (area * kTwelfth);
+                const double K_ij = area * (g.dNdx[a] * g.dNdx[j] + g.dNdy[a] * g.dNdy[j]);
+                const double C_ij = area3 * ugN[j] + P.skew_coef * div_w * M_ij;
+                const double S_ij = area * tau_supg * ugN[a] * ugN[j];
+                const double Ms_ij = area3 * tau_supg * ugN[a];
+                rec[(3 * a + j) * S] = P.a0 * (M_ij + Ms_ij) + nu * K_ij + C_ij + S_ij;
+                f_u += (M_ij + Ms_ij) * u_h[j];
+                f_v += (M_ij + Ms_ij) * v_h[j];
+            }
+            const double tw = area3 + area * tau_supg * ugN[a];
+            rec[(9 + a) * S] = f_u - tw * dpdx;
+            rec[(12 + a) * S] = f_v - tw * dpdy;
+        }
+        rec[15 * S] = area3;
+    }
+    __syncthreads();
+    const int p0 = rp[b.r0], p1 = rp[b.r1];
+    const unsigned short* code = tv.ecode + 3 * (size_t)b.i0;
+    auto entry = [&](int p, int c0, int c1) {
+        double v = 0.0;
+        for (int c = c0; c < c1; ++c) {
+            const int q = code[c];
+            v += et_rec[(3 * ((q >> 2) & 3) + (q & 3)) * S + (q >> 4)];
+        }
+        A_val[p] = v;
+    };
+    for (int p = p0 + threadIdx.x; p < p1; p += kEtThreads)
+        entry(p, tv.eoff[p], p + 1 < p1 ? (int)tv.eoff[p + 1] : 3 * (b.i1 - b.i0));
+    if (with_bc) __syncthreads();   // the Dirichlet rows below follow the entries' values
+    for (int i = b.r0 + threadIdx.x; i < b.r1; i += kEtThreads) {
+        double f_u = 0.0, f_v = 0.0, m = 0.0;
+        for (int s = tv.inc_ptr[i]; s < tv.inc_ptr[i + 1]; ++s) {
+            const int q = tv.rcode[s], le = q >> 2, a = q & 3;
+            f_u += et_rec[(9 + a) * S + le];
+            f_v += et_rec[(12 + a) * S + le];
+            m += et_rec[15 * S + le];
+        }
+        mass[i] = m;
+        const int t = tag[i];
+        if (with_bc && momentum_dirichlet(t, bc)) {
+            for (int q = rp[i]; q < rp[i + 1]; ++q) A_val[q] = (ci[q] == i) ? 1.0 : 0.0;
+            f_u = momentum_bc_u(t, y[i], u_max, H, bc);
+            f_v = 0.0;
+        }
+        rhs_u[i] = f_u;
+        rhs_v[i] = f_v;
+    }
 }
 
 // Dirichlet rows of the momentum system alone (k_apply_bc_momentum, fem_kernels.cuh:411-453);
@@ -367,6 +478,174 @@ k_pressure_rows(int n, int nnz, const int* __restrict__ ev, const double* __rest
     rhs_p[i] = rhs_row;
 }
 
+// Scalar gradient on element tiles: grad f and the weight (area / 3) sqrt(s) of every element
+// once, then the rows. Against the row gather 9.4 -> 6.3 us at 22.5k vertices, 8.3 -> 6.1 us at 8k,
+// 29.9 -> 31.0 us at 402k, 269 -> 389 us at 4.2M: the tile's plan is as many bytes as it saves, so
+// the form pays only while the mesh is latency (kGradTileRows).
+constexpr int kGradTileRows = 150'000;
+
+__global__ void __launch_bounds__(kEtThreads)
+k_scalar_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
+                        const double* __restrict__ y, const double* __restrict__ f, const double* __restrict__ elem_s,
+                        double* __restrict__ gx_out, double* __restrict__ gy_out) {
+    extern __shared__ __align__(16) double et_rec[];   // [3][tv.stride]
+    const EtBlock b = et_block(tv, n);
+    const int S = tv.stride;
+    CFA_GRID_DEP();
+    for (int le = threadIdx.x; le < b.ne; le += kEtThreads) {
+        int nd[3];
+        load_elem(ev, tv.elems[b.i0 + le], nd);
+        const double es = elem_s ? elem_s[tv.elems[b.i0 + le]] : 1.0;
+        const double x0 = x[nd[0]], y0 = y[nd[0]], x1 = x[nd[1]], y1 = y[nd[1]], x2 = x[nd[2]], y2 = y[nd[2]];
+        const double f0 = f[nd[0]], f1 = f[nd[1]], f2 = f[nd[2]];
+        const double detJ = (x1 - x0) * (y2 - y0) - (x2 - x0) * (y1 - y0);
+        const double area = 0.5 * fabs(detJ);
+        double gx = 0.0, gy = 0.0, w = 0.0;
+        if (!(area < 1.0e-14)) {
+            const double inv2A = 1.0 / (2.0 * area);
+            w = (elem_s ? sqrt(es) : 1.0) * area / 3.0;
+            gx = (f0 * (y1 - y2) + f1 * (y2 - y0) + f2 * (y0 - y1)) * inv2A;
+            gy = (f0 * (x2 - x1) + f1 * (x0 - x2) + f2 * (x1 - x0)) * inv2A;
+        }
+        et_rec[le] = gx;
+        et_rec[S + le] = gy;
+        et_rec[2 * S + le] = w;
+    }
+    __syncthreads();
+    for (int i = b.r0 + threadIdx.x; i < b.r1; i += kEtThreads) {
+        double sx = 0.0, sy = 0.0;
+        for (int s = tv.inc_ptr[i]; s < tv.inc_ptr[i + 1]; ++s) {
+            const int le = tv.rcode[s] >> 2;
+            const double w = et_rec[2 * S + le];
+            sx = __fma_rn(w, et_rec[le], sx);
+            sy = __fma_rn(w, et_rec[S + le], sy);
+        }
+        gx_out[i] = sx;
+        gy_out[i] = sy;
+    }
+}
+
+// Pressure rows on element tiles, 19 doubles an element: the symmetric K (6), grad N (6), w, 1 + s,
+// the right-hand side of each vertex (3), area / 3 and div u. The weights enter the sums by fused
+// multiply-adds, as in the row gather. Bound by shared memory: seven 8-byte reads a contribution,
+// 2.6 contributions an entry, and the records limit the blocks per SM. Staging the codes in shared
+// memory and loading offsets ahead was slower (152 us), as were blocks of 384 threads (177 us).
+// Against the row gather: 367 -> 148 us at 402k vertices (190 MB, 1.3 TB/s), 3713 -> 1650 us at 4.2M,
+// 32.2 -> 10.8 us at 22.5k, 25.1 -> 9.0 us at 8k.
+__global__ void __launch_bounds__(kEtThreads)
+k_pressure_tiles(ElemTileView tv, int n, int nnz, const int* __restrict__ ev, const double* __restrict__ x,
+                 const double* __restrict__ y, const int* __restrict__ tag, const int* __restrict__ rp,
+                 const int* __restrict__ ci, const double* __restrict__ us, const double* __restrict__ vs,
+                 const double* __restrict__ p_old, const double* __restrict__ gpx, const double* __restrict__ gpy,
+                 const double* __restrict__ mass, const double* __restrict__ elem_s, double dt, double rho,
+                 double stab, int with_bc, OutletBc bc, double* __restrict__ Kp_val, double* __restrict__ rhs_p,
+                 double* __restrict__ div_num, double* __restrict__ dp, double* __restrict__ oss_val,
+                 double* __restrict__ inv_m) {
+    extern __shared__ __align__(16) double et_rec[];   // [19][tv.stride]
+    const EtBlock b = et_block(tv, n);
+    const int S = tv.stride;
+    const bool want_oss = oss_val != nullptr;
+    CFA_GRID_DEP();
+    for (int le = threadIdx.x; le < b.ne; le += kEtThreads) {
+        int nd[3];
+        load_elem(ev, tv.elems[b.i0 + le], nd);
+        const double es = stab > 0.0 || want_oss ? elem_s[tv.elems[b.i0 + le]] : 0.0;
+        const Geom g = elem_geom(nd, x, y);
+        double* rec = et_rec + le;
+        if (!g.ok) {
+#pragma unroll
+            for (int q = 0; q < 19; ++q) rec[q * S] = 0.0;
+            continue;
+        }
+        const double area = g.area;
+        const double div_u = us[nd[0]] * g.dNdx[0] + us[nd[1]] * g.dNdx[1] + us[nd[2]] * g.dNdx[2]
+                           + vs[nd[0]] * g.dNdy[0] + vs[nd[1]] * g.dNdy[1] + vs[nd[2]] * g.dNdy[2];
+        const double rs = sqrt(es);
+        double s = 0.0, sx = 0.0, sy = 0.0, gx = 0.0, gy = 0.0;
+        if (stab > 0.0) {
+            s = es;
+            gx = p_old[nd[0]] * g.dNdx[0] + p_old[nd[1]] * g.dNdx[1] + p_old[nd[2]] * g.dNdx[2];
+            gy = p_old[nd[0]] * g.dNdy[0] + p_old[nd[1]] * g.dNdy[1] + p_old[nd[2]] * g.dNdy[2];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const double im = 1.0 / fmax(mass[nd[q]], 1.0e-14);
+                sx = __fma_rn(gpx[nd[q]], im, sx);
+                sy = __fma_rn(gpy[nd[q]], im, sy);
+            }
+            sx *= rs / 3.0;
+            sy *= rs / 3.0;
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+#pragma unroll
+            for (int j = a; j < 3; ++j)   // 00 01 02 11 12 22
+                rec[(a + j + (a > 0 ? 1 : 0)) * S] = area * (g.dNdx[a] * g.dNdx[j] + g.dNdy[a] * g.dNdy[j]);
+            rec[(6 + a) * S] = g.dNdx[a];
+            rec[(9 + a) * S] = g.dNdy[a];
+            // rhs - (s area (grad N . grad p) - area (grad N . the projection)), rounded explicitly:
+            // the PPE alone and the fused system give the same bits whatever the compiler contracts
+            const double stab_i =
+                __fma_rn(s * area, __fma_rn(g.dNdx[a], gx, __dmul_rn(g.dNdy[a], gy)),
+                         -__dmul_rn(area, __fma_rn(g.dNdx[a], sx, __dmul_rn(g.dNdy[a], sy))));
+            rec[(14 + a) * S] = __fma_rn(-(rho / dt) * (area / 3.0), div_u, -stab_i);
+        }
+        rec[12 * S] = rs * area / 3.0;
+        rec[13 * S] = 1.0 + s;
+        rec[17 * S] = area / 3.0;
+        rec[18 * S] = div_u;
+    }
+    __syncthreads();
+    double *Bx = oss_val, *By = oss_val + (size_t)nnz, *BTx = oss_val + 2 * (size_t)nnz, *BTy = oss_val + 3 * (size_t)nnz;
+    const int p0 = rp[b.r0], p1 = rp[b.r1];
+    const unsigned short* code = tv.ecode + 3 * (size_t)b.i0;
+    auto entry = [&](int p, int c0, int c1) {
+        double k = 0.0, bx = 0.0, by = 0.0, tx = 0.0, ty = 0.0;
+        for (int c = c0; c < c1; ++c) {
+            const int q = code[c], a = (q >> 2) & 3, j = q & 3;
+            const double* rec = et_rec + (q >> 4);
+            k = __fma_rn(rec[13 * S], rec[(a + j + (a > 0 && j > 0 ? 1 : 0)) * S], k);
+            if (want_oss) {
+                // B_ij = sum_K w_K grad N_j|K (row i, column j); B^T_ij = B_ji = sum_K w_K grad N_i|K
+                const double w = rec[12 * S];
+                bx = __fma_rn(w, rec[(6 + j) * S], bx);
+                by = __fma_rn(w, rec[(9 + j) * S], by);
+                tx = __fma_rn(w, rec[(6 + a) * S], tx);
+                ty = __fma_rn(w, rec[(9 + a) * S], ty);
+            }
+        }
+        if (with_bc) {   // a Dirichlet column; its own row is written below
+            const int col = ci[p];
+            if (pressure_dirichlet(col, tag[col], bc)) k = 0.0;
+        }
+        Kp_val[p] = k;
+        if (want_oss) {
+            Bx[p] = bx;
+            By[p] = by;
+            BTx[p] = tx;
+            BTy[p] = ty;
+        }
+    };
+    for (int p = p0 + threadIdx.x; p < p1; p += kEtThreads)
+        entry(p, tv.eoff[p], p + 1 < p1 ? (int)tv.eoff[p + 1] : 3 * (b.i1 - b.i0));
+    if (with_bc) __syncthreads();   // the Dirichlet rows below follow the entries' values
+    for (int i = b.r0 + threadIdx.x; i < b.r1; i += kEtThreads) {
+        double r = 0.0, d = 0.0;
+        for (int s = tv.inc_ptr[i]; s < tv.inc_ptr[i + 1]; ++s) {
+            const int q = tv.rcode[s], le = q >> 2;
+            r += et_rec[(14 + (q & 3)) * S + le];
+            d = __fma_rn(et_rec[17 * S + le], et_rec[18 * S + le], d);
+        }
+        if (want_oss) inv_m[i] = 1.0 / fmax(mass[i], 1.0e-14);
+        div_num[i] = d;
+        if (with_bc && pressure_dirichlet(i, tag[i], bc)) {
+            for (int q = rp[i]; q < rp[i + 1]; ++q) Kp_val[q] = (ci[q] == i) ? 1.0 : 0.0;
+            r = 0.0;
+            if (dp) dp[i] = 0.0;
+        }
+        rhs_p[i] = r;
+    }
+}
+
 // k_apply_bc_pressure (fem_kernels.cuh:460-490) alone; with mean removal first when pinned
 // (k_sum / k_subtract_mean, :493-510, summed here in a fixed order).
 __global__ void k_pressure_bc(int n, const int* __restrict__ tag, const int* __restrict__ rp,
@@ -414,6 +693,15 @@ static cfa_status mean_removal_sums(cfa_ctx* ctx, int n, const double* rhs, cons
     return CFA_OK;
 }
 
+static void allow_et_kernels() {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaFuncSetAttribute(k_momentum_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, kEtMaxSmem);
+        cudaFuncSetAttribute(k_pressure_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, kEtMaxSmem);
+        cudaFuncSetAttribute(k_scalar_gradient_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, kEtMaxSmem);
+    });
+}
+
 }  // namespace cfa
 
 using namespace cfa;
@@ -444,9 +732,15 @@ cfa_status cfa_assemble_momentum_nu(cfa_ctx* ctx, const cfa_mesh* m, const doubl
     CFA_ARG(!bcp || (u && v));
     MomParams P{prm->dt, prm->nu, prm->rho, prm->a0, prm->a1, prm->a2, prm->c1, prm->c2, prm->tau_time, prm->skew_coef};
     const double u_max = bcp ? bcp->u_max : 0.0, H = bcp ? bcp->H : 1.0;
-    CFA_LAUNCH(ctx, k_momentum_rows, ceil_div(m->n, kThreads), kThreads, kMomSmem, m->n, m->ev, m->x, m->y, m->tag,
-               m->inc_ptr.p, m->inc.p, m->pos.p, m->rp, m->ci, u_old, v_old, u_prev, v_prev, p_old, nu_node, P,
-               bcp ? 1 : 0, u_max, H, m->bc, A_val, rhs_u, rhs_v, mass);
+    allow_et_kernels();
+    if (m->et.ok)
+        CFA_LAUNCH(ctx, k_momentum_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 16), m->tiles(), m->n, m->ev,
+                   m->x, m->y, m->tag, m->rp, m->ci, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, bcp ? 1 : 0, u_max, H, m->bc,
+                   A_val, rhs_u, rhs_v, mass);
+    else
+        CFA_LAUNCH(ctx, k_momentum_rows, ceil_div(m->n, kThreads), kThreads, kMomSmem, m->n, m->ev, m->x, m->y, m->tag,
+                   m->inc_ptr.p, m->inc.p, m->pos.p, m->rp, m->ci, u_old, v_old, u_prev, v_prev, p_old, nu_node, P,
+                   bcp ? 1 : 0, u_max, H, m->bc, A_val, rhs_u, rhs_v, mass);
     if (bcp)   // solution values on Dirichlet nodes after the rows (u may alias u_old)
         CFA_LAUNCH(ctx, k_momentum_bc, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->tag, m->y, m->rp, m->ci,
                    u_max, H, m->bc, 0, A_val, rhs_u, rhs_v, u, v);
@@ -487,8 +781,13 @@ cfa_status cfa_scalar_gradient(cfa_ctx* ctx, const cfa_mesh* m, const double* f,
                                double* gy) {
     CFA_ENTER(ctx);
     CFA_ARG(m && f && gx && gy);
-    CFA_LAUNCH(ctx, k_scalar_gradient_rows, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y,
-               m->inc_ptr.p, m->inc.p, f, elem_s, gx, gy);
+    allow_et_kernels();
+    if (m->et.ok && m->n <= kGradTileRows)
+        CFA_LAUNCH(ctx, k_scalar_gradient_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 3), m->tiles(), m->n,
+                   m->ev, m->x, m->y, f, elem_s, gx, gy);
+    else
+        CFA_LAUNCH(ctx, k_scalar_gradient_rows, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y,
+                   m->inc_ptr.p, m->inc.p, f, elem_s, gx, gy);
     CFA_CHECK_LAUNCH();
     return CFA_OK;
 }
@@ -505,10 +804,16 @@ static cfa_status assemble_pressure(cfa_ctx* ctx, const cfa_mesh* m, const doubl
     std::call_once(press_once, [] {
         cudaFuncSetAttribute(k_pressure_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPressSmem);
     });
-    CFA_LAUNCH(ctx, k_pressure_rows, ceil_div(m->n, kPressThreads), kPressThreads, kPressSmem, m->n, m->nnz, m->ev,
-               m->x, m->y, m->tag,
-               m->inc_ptr.p, m->inc.p, m->pos.p, m->rp, m->ci, us, vs, p_old, gpx, gpy, mass, elem_s, dt, rho,
-               stab, (apply_bc && !split) ? 1 : 0, m->bc, Kp, rhs, div, dp, oss_val, inv_m);
+    allow_et_kernels();
+    const int with_bc = (apply_bc && !split) ? 1 : 0;
+    if (m->et.ok)
+        CFA_LAUNCH(ctx, k_pressure_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 19), m->tiles(), m->n,
+                   m->nnz, m->ev, m->x, m->y, m->tag, m->rp, m->ci, us, vs, p_old, gpx, gpy, mass, elem_s, dt, rho, stab, with_bc,
+                   m->bc, Kp, rhs, div, dp, oss_val, inv_m);
+    else
+        CFA_LAUNCH(ctx, k_pressure_rows, ceil_div(m->n, kPressThreads), kPressThreads, kPressSmem, m->n, m->nnz, m->ev,
+                   m->x, m->y, m->tag, m->inc_ptr.p, m->inc.p, m->pos.p, m->rp, m->ci, us, vs, p_old, gpx, gpy, mass,
+                   elem_s, dt, rho, stab, with_bc, m->bc, Kp, rhs, div, dp, oss_val, inv_m);
     if (split) {
         double* sums = ctx->d_part;   // after the partials region
         CFA_PROPAGATE(ensure_partials(ctx, 2 * (size_t)row_grid(ctx, m->n, 1) + 4));

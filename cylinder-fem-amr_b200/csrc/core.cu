@@ -164,6 +164,106 @@ static cfa_status build_incidence(cfa_ctx* ctx, int n, int ne, const int* d_ev, 
     return CFA_OK;
 }
 
+// Element tiles (elemtile.cuh), one block per tile: its incidences' elements sorted and made unique,
+// the local element of every incidence, and every CSR entry's contributions in incidence order.
+// flags[0]: the largest element count, flags[1]: a tile with too many incidences.
+__global__ void __launch_bounds__(kEtThreads)
+k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __restrict__ inc,
+             const int* __restrict__ pos, const int* __restrict__ rp, int* __restrict__ elems,
+             int* __restrict__ count, unsigned short* __restrict__ rcode, unsigned short* __restrict__ ecode,
+             unsigned short* __restrict__ eoff, int* __restrict__ flags) {
+    constexpr int kItems = kEtMaxInc / kEtThreads;
+    using Sort = cub::BlockRadixSort<int, kEtThreads, kItems>;
+    using Scan = cub::BlockScan<int, kEtThreads>;
+    __shared__ union {
+        typename Sort::TempStorage sort;
+        typename Scan::TempStorage scan;
+    } tmp;
+    __shared__ int uniq[kEtMaxInc];
+    __shared__ int last_key[kEtThreads];
+    __shared__ unsigned short rc[kEtMaxInc];
+    const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+    const int i0 = inc_ptr[r0], m = inc_ptr[r1] - i0;
+    if (m > kEtMaxInc) {
+        if (threadIdx.x == 0) {
+            flags[1] = 1;
+            count[blockIdx.x] = 0;
+        }
+        return;
+    }
+    int key[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int s = threadIdx.x * kItems + k;
+        key[k] = s < m ? inc[i0 + s] >> 2 : 0x7fffffff;
+    }
+    Sort(tmp.sort).Sort(key);
+    last_key[threadIdx.x] = key[kItems - 1];
+    __syncthreads();
+    int first[kItems], rank[kItems], total = 0;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int prev = k > 0 ? key[k - 1] : threadIdx.x > 0 ? last_key[threadIdx.x - 1] : -1;
+        first[k] = key[k] != prev && key[k] != 0x7fffffff ? 1 : 0;
+    }
+    Scan(tmp.scan).ExclusiveSum(first, rank, total);
+#pragma unroll
+    for (int k = 0; k < kItems; ++k)
+        if (first[k]) {
+            uniq[rank[k]] = key[k];
+            elems[i0 + rank[k]] = key[k];
+        }
+    if (threadIdx.x == 0) {
+        count[blockIdx.x] = total;
+        atomicMax(&flags[0], total);
+    }
+    __syncthreads();
+    for (int s = threadIdx.x; s < m; s += kEtThreads) {
+        const int v = inc[i0 + s], e = v >> 2;
+        int lo = 0, hi = total - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (uniq[mid] < e) lo = mid + 1;
+            else hi = mid;
+        }
+        rc[s] = (unsigned short)((lo << 2) | (v & 3));
+        rcode[i0 + s] = rc[s];
+    }
+    __syncthreads();
+    // row by row: an entry's contributions are the (incidence, column) pairs whose position it is
+    for (int i = r0 + threadIdx.x; i < r1; i += kEtThreads) {
+        const int s0 = inc_ptr[i] - i0, s1 = inc_ptr[i + 1] - i0;
+        int cur = 3 * s0;
+        for (int p = rp[i]; p < rp[i + 1]; ++p) {
+            eoff[p] = (unsigned short)cur;
+            for (int s = s0; s < s1; ++s)
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+                    if (pos[3 * (size_t)(i0 + s) + b] == p)
+                        ecode[3 * (size_t)i0 + cur++] =
+                            (unsigned short)(((rc[s] >> 2) << 4) | ((rc[s] & 3) << 2) | b);
+        }
+    }
+}
+
+// The mesh's element tiles; flags (2 ints, zeroed) are read back by the caller.
+static cudaError_t plan_elem_tiles(cfa_ctx* ctx, cfa_mesh* m, int nnz, int* flags) {
+    ElemTiles& T = m->et;
+    T.rows = elem_tile_rows(m->n, ctx->num_sms);
+    T.ntiles = ceil_div(m->n, T.rows);
+    const size_t inc = 3 * (size_t)m->ne;
+    cudaError_t e = T.elems.ensure(inc);
+    if (e == cudaSuccess) e = T.count.ensure(T.ntiles);
+    if (e == cudaSuccess) e = T.rcode.ensure(inc);
+    if (e == cudaSuccess) e = T.ecode.ensure(3 * inc);
+    if (e == cudaSuccess) e = T.eoff.ensure((size_t)nnz + 1);
+    if (e != cudaSuccess) return e;
+    CFA_LAUNCH(ctx, k_elem_tiles, T.ntiles, kEtThreads, 0, m->n, T.rows, (const int*)m->inc_ptr.p,
+               (const int*)m->inc.p, (const int*)m->pos.p, m->rp, T.elems.p, T.count.p, T.rcode.p,
+               T.ecode.p, T.eoff.p, flags);
+    return cudaGetLastError();
+}
+
 }  // namespace cfa
 
 using namespace cfa;
@@ -316,20 +416,25 @@ cfa_status cfa_mesh_create(cfa_ctx* ctx, int n, int ne, const int* d_ev, const d
     m->ci = d_ci;
     cfa_status s = build_incidence(ctx, n, ne, d_ev, m->inc_ptr, m->inc);
     if (s != CFA_OK) { delete m; return s; }
-    DevBuf<int> err;
+    DevBuf<int> err;   // a missing entry, then the element tiles' flags
+    int h_nnz = 0;
     cudaError_t e = m->pos.ensure(9 * (size_t)ne);
-    if (e == cudaSuccess) e = err.ensure(1);
-    if (e == cudaSuccess) e = cudaMemsetAsync(err.p, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess) e = err.ensure(3);
+    if (e == cudaSuccess) e = cudaMemsetAsync(err.p, 0, 3 * sizeof(int), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_nnz, d_rp + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) { delete m; return set_error(ctx, CFA_CUDA_ERROR, cudaGetErrorString(e), __FILE__, __LINE__); }
     ctx->launches++;
     k_scatter_positions<<<ceil_div(n, kThreads), kThreads, 0, ctx->stream>>>(n, d_ev, m->inc_ptr.p, m->inc.p, d_rp,
                                                                                d_ci, m->pos.p, err.p);
-    int h_nnz = 0, h_err = 0;
-    e = cudaMemcpyAsync(&h_nnz, d_rp + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    e = plan_elem_tiles(ctx, m, h_nnz, err.p + 1);
+    int h_err[3] = {0, 0, 0};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_err, err.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) { delete m; return set_error(ctx, CFA_CUDA_ERROR, cudaGetErrorString(e), __FILE__, __LINE__); }
-    if (h_err) { delete m; return set_error(ctx, CFA_BAD_ARG, "element edge missing from the CSR pattern", __FILE__, __LINE__); }
+    if (h_err[0]) { delete m; return set_error(ctx, CFA_BAD_ARG, "element edge missing from the CSR pattern", __FILE__, __LINE__); }
+    m->et.max_elems = (h_err[1] + 3) & ~3;
+    m->et.ok = !h_err[2] && et_smem_bytes(m->et, kEtMaxRec) <= kEtMaxSmem;
     m->nnz = h_nnz;
     *out = m;
     return CFA_OK;

@@ -4,6 +4,7 @@
 // find_csr_index of src/cfa/fem_kernels.cuh:12-28).
 #pragma once
 
+#include "elemtile.cuh"
 #include "internal.cuh"
 
 namespace cfa {
@@ -34,5 +35,9 @@ struct cfa_mesh {
     cfa::DevBuf<int> inc_ptr;    // [n + 1]
     cfa::DevBuf<int> inc;        // [3 ne]: element << 2 | local vertex, ascending element per node
     cfa::DevBuf<int> pos;        // [9 ne]: pos[3 s + b] = CSR index of (node of s, vertex b of its element)
+    cfa::ElemTiles et;           // elements of blocks of rows (elemtile.cuh)
+    cfa::ElemTileView tiles() const {
+        return {et.rows, et.ntiles, et.max_elems, et.elems.p, et.count.p, inc_ptr.p, et.rcode.p, et.ecode.p, et.eoff.p};
+    }
     cfa::OutletBc bc;
 };

@@ -1,0 +1,111 @@
+"""Assembly on element tiles (a block's elements computed once) and its row-gather form for tiles
+too large, against the oracle: meshes of one element to several tile heights, orders that scatter
+a tile's elements, and a node of more elements than a tile holds."""
+import numpy as np
+import pytest
+
+import fixtures as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _shuffled(m, seed=1):
+    """Vertices and elements in random order: a tile of rows touches almost only its own elements."""
+    rng = np.random.default_rng(seed)
+    perm, eperm = rng.permutation(m.n), rng.permutation(m.ne)
+    new = np.empty_like(perm)
+    new[perm] = np.arange(m.n)
+    return F.Mesh(m.x[perm].copy(), m.y[perm].copy(), m.tag[perm].copy(),
+                  new[m.tri][eperm].astype(np.int32), m.gen[eperm].copy())
+
+
+def _wheel(spokes):
+    """A disc of `spokes` elements around vertex 0, its rim in [0, 1] x [0, 1]."""
+    th = 2 * np.pi * np.arange(spokes) / spokes
+    x = np.concatenate([[0.5], 0.5 + 0.5 * np.cos(th)])
+    y = np.concatenate([[0.5], 0.5 + 0.5 * np.sin(th)])
+    k = np.arange(spokes)
+    tri = np.stack([np.zeros(spokes, np.int64), 1 + k, 1 + (k + 1) % spokes], 1).astype(np.int32)
+    tag = np.zeros(spokes + 1, np.int32)
+    tag[1::7], tag[2::7], tag[3::11] = F.BC_INLET, F.BC_OUTLET, F.BC_WALL
+    return F.Mesh(x, y, tag, tri, np.zeros(spokes, np.int32))
+
+
+def _one():
+    return F.Mesh(np.array([0.0, 1.0, 0.3]), np.array([0.0, 0.2, 0.9]), np.array([0, 2, 1], np.int32),
+                  np.array([[0, 1, 2]], np.int32), np.zeros(1, np.int32))
+
+
+CASES = {
+    "one": _one,
+    "tiny": lambda: F.make_mesh("tiny"),
+    "small": lambda: F.make_mesh("small"),
+    "small_shuffled": lambda: _shuffled(F.make_mesh("small")),
+    "c0_rows64": lambda: F.make_mesh("c0"),
+    "medium_rows96": lambda: F.make_mesh("medium"),
+    "wheel_127": lambda: _wheel(127),
+    "wheel_1200": lambda: _wheel(1200),          # one tile with nearly all of a block's shared memory
+    "wheel_2000_gather": lambda: _wheel(2000),   # records beyond it: the row gathers
+    "wheel_3100_gather": lambda: _wheel(3100),   # incidences beyond the plan's sort
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("outlet_dirichlet", [0, 1])
+def test_assembly_matches_the_oracle(name, outlet_dirichlet):
+    import torch
+    import cfa_b200 as cfa
+    from oracle import oracle as O
+    m = CASES[name]()
+    ctx = cfa.default_context()
+    rp, ci = O.csr_build(m.n, m.elem_v)
+    dm = cfa.DeviceMesh(ctx, m, torch.from_numpy(rp).to("cuda"), torch.from_numpy(ci).to("cuda"))
+    pin = int(np.flatnonzero(m.tag == F.BC_OUTLET)[0])
+    if outlet_dirichlet:
+        dm.set_outlet(1, pin, 1.25)
+    n, nnz = m.n, len(ci)
+    u, v, p = (F.fourier_field(m.x, m.y, 1), F.fourier_field(m.x, m.y, 2), 0.3 * F.fourier_field(m.x, m.y, 3))
+    up, vp = 0.9 * u, 1.1 * v
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float64)).to("cuda")
+    z = lambda k: torch.full((k,), float("nan"), dtype=torch.float64, device="cuda")
+    # momentum without its boundary rows, then the library's own boundary rows on both
+    A, ru, rv, mass = z(nnz), z(n), z(n), z(n)
+    prm = cfa.bdf2_params()
+    cfa.assemble_momentum(ctx, dm, t(u), t(v), t(up), t(vp), t(p), prm, A, ru, rv, mass)
+    oA, oru, orv, omass = O.assemble_momentum(m, rp, ci, u, v, up, vp, p, O.bdf2_params())
+    # every value is a sum of at most a few hundred terms of its own size in the same order; the
+    # element formulas differ by reciprocals and contractions: a few hundred roundings of 1.1e-16
+    for got, want in ((A, oA), (ru, oru), (rv, orv), (mass, omass)):
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-12 * np.abs(want).max()
+    A2, ru2, rv2, mass2, uu, vv = z(nnz), z(n), z(n), z(n), t(u), t(v)
+    cfa.assemble_momentum(ctx, dm, t(u), t(v), t(up), t(vp), t(p), prm, A2, ru2, rv2, mass2, uu, vv, u_max=1.5)
+    uu1, vv1 = t(u), t(v)
+    cfa.apply_bc_momentum(ctx, dm, A, ru, rv, uu1, vv1, 1.5)
+    for a, b in ((A, A2), (ru, ru2), (rv, rv2), (uu, uu1), (vv, vv1)):
+        assert torch.equal(a, b)
+    # pressure: values, right-hand side and OSS operator without boundary rows, then with them
+    dt = 2e-3 / 3
+    s = O.oss_weights(m, u, v, dt, 1.0, 1e-3, 0.3)
+    gx, gy = z(n), z(n)
+    cfa.scalar_gradient(ctx, dm, t(p), t(s), gx, gy)
+    ogx, ogy = O.scalar_gradient(m, p, s)
+    for got, want in ((gx, ogx), (gy, ogy)):
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-12 * max(np.abs(ogx).max(), np.abs(ogy).max())
+    K, rhs, div = z(nnz), z(n), z(n)
+    cfa.assemble_ppe(ctx, dm, t(u), t(v), t(p), t(ogx), t(ogy), t(omass), t(s), dt, 1.0, 0.3, K, rhs, div,
+                     apply_bc=False)
+    oK, orhs, odiv = O.assemble_ppe(m, rp, ci, u, v, p, ogx, ogy, omass, s, dt, 1.0, 0.3)
+    for got, want in ((K, oK), (rhs, orhs), (div, odiv)):
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-11 * np.abs(want).max()
+    oss, im = z(4 * nnz), z(n)
+    cfa.assemble_oss(ctx, dm, t(s), t(omass), oss, im)
+    ooss, oim = O.assemble_oss(m, rp, ci, s, omass)
+    for got, want in ((oss, ooss), (im, oim)):
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-12 * np.abs(want).max()
+    K2, rhs2, div2, dp2, oss2, im2 = z(nnz), z(n), z(n), t(p), z(4 * nnz), z(n)
+    cfa.assemble_pressure_system(ctx, dm, t(u), t(v), t(p), t(ogx), t(ogy), t(omass), t(s), dt, 1.0, 0.3, K2, rhs2,
+                                 div2, dp2, oss2, im2)
+    dp1 = t(p)
+    cfa.apply_bc_pressure(ctx, dm, K, rhs, dp1, t(omass))
+    for a, b in ((K, K2), (rhs, rhs2), (div, div2), (dp1, dp2), (oss, oss2), (im, im2)):
+        assert torch.equal(a, b)
