@@ -1076,6 +1076,182 @@ static void vct(cfa_ctx* ctx, bool dry, const TiledCsr& M, int* err, const T* di
 }
 
 // ---------------------------------------------------------------------------------------------
+// level 0's sweeps in pairs over ring tiles (ring.cuh)
+// ---------------------------------------------------------------------------------------------
+// RING_PRE: x = VC_PRE of b, out = b - A x; RING_PREC: the same with the first iterate c = x given;
+// RING_JAC: out = two Jacobi sweeps from x (RZ: with the CG's dots of out). xout: RING_PRE(C)'s x.
+// Bound by latency at the sizes that take it (ring_rows, ring.cu): one round of gathers, then two
+// sweeps from shared memory, in place of two kernels. 8k vertices: a pair of kernels 7.4 us -> 4.1 us,
+// the FP64 V-cycle 28.7 -> 21.0 us; 37k: 35.2 -> 31.7 us.
+enum RingOp { RING_PRE = 0, RING_PREC = 1, RING_JAC = 2 };
+
+// One row's sum over its entries in order, the loads of a batch ahead of its sums
+template <class V, class T>
+__device__ __forceinline__ T ring_row(const unsigned short* rr, const unsigned short* cs, const V* vv, const T* vec,
+                                      int lr) {
+    T s = (T)0;
+    const int end = rr[lr + 1];
+    for (int e0 = rr[lr]; e0 < end; e0 += kGatherBatch) {
+        T a[kGatherBatch], g[kGatherBatch];
+#pragma unroll
+        for (int u = 0; u < kGatherBatch; ++u)
+            if (e0 + u < end) {
+                a[u] = (T)vv[e0 + u];
+                g[u] = vec[cs[e0 + u]];
+            }
+#pragma unroll
+        for (int u = 0; u < kGatherBatch; ++u)
+            if (e0 + u < end) s += a[u] * g[u];
+    }
+    return s;
+}
+
+template <int OP, class V, class T, class B, class O, bool RZ>
+__global__ void __launch_bounds__(kRingThreads)
+k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* __restrict__ b, const T* __restrict__ x,
+       T* __restrict__ xout, O* __restrict__ out, const int* __restrict__ done, RzFuse rzf) {
+    extern __shared__ __align__(128) unsigned char rsmem[];
+    __shared__ uint64_t bar;
+    __shared__ int abort_flag;
+    const RingSmem L = ring_smem_layout(rv.max_rows, rv.max_local, rv.max_ne, (int)sizeof(V), (int)sizeof(T));
+    const unsigned short* rr = reinterpret_cast<const unsigned short*>(rsmem + L.rp);
+    const unsigned short* cs = reinterpret_cast<const unsigned short*>(rsmem + L.ci);
+    const V* vv = reinterpret_cast<const V*>(rsmem + L.v);
+    T* xs = reinterpret_cast<T*>(rsmem + L.x);
+    T* ys = reinterpret_cast<T*>(rsmem + L.y);
+    T* bs = reinterpret_cast<T*>(rsmem + L.b);
+    T* od = reinterpret_cast<T*>(rsmem + L.od);
+    int* hl = reinterpret_cast<int*>(rsmem + L.hl);
+    double dots[2] = {0.0, 0.0};
+    unsigned phase = 0u;
+    bool first = true;
+    for (int t = blockIdx.x; t < rv.ntiles; t += gridDim.x) {
+        const RingMeta m = rv.meta[t];
+        const int r0 = t * rv.rows, nr = min(rv.rows, rv.n - r0), R = nr + m.h1, N = R + m.h2;
+        if (threadIdx.x == 0) {
+            if (first) {
+                mbar_init(&bar, 1);
+                mbar_fence_init();
+                abort_flag = 0;
+            } else {
+                fence_proxy_async();
+            }
+            const unsigned nb_rp = (unsigned)align16(2LL * (R + 1)), nb_ci = (unsigned)align16(2LL * m.ne),
+                           nb_v = (unsigned)align16((long long)sizeof(V) * m.ne);
+            mbar_expect_tx(&bar, nb_rp + nb_ci + nb_v);
+            bulk_g2s(rsmem + L.rp, rv.rp + (size_t)t * rv.rp_stride, nb_rp, &bar);
+            bulk_g2s(rsmem + L.ci, rv.ci + m.e0, nb_ci, &bar);
+            bulk_g2s(rsmem + L.v, rv.v + m.e0, nb_v, &bar);
+        }
+        for (int k = threadIdx.x; k < m.h1 + m.h2; k += kRingThreads) hl[k] = rv.halo[(size_t)t * kRingHalo + k];
+        if (first) {
+            // the tiles belong to the setup: their copies go out before the wait (tiled.cuh)
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            CFA_GRID_DEP();
+        }
+        __syncthreads();
+        if (first && done && *done) {
+            if (threadIdx.x == 0) mbar_wait(&bar, 0u);
+            return;
+        }
+        for (int lr = threadIdx.x; lr < N; lr += kRingThreads) {
+            const int j = lr < nr ? r0 + lr : hl[lr - nr];
+            if (OP == RING_PRE) {
+                const T o = omega * dinv[j], bj = (T)b[j];
+                xs[lr] = mul_rn(o, bj);
+                if (lr < R) {
+                    od[lr] = o;
+                    bs[lr] = bj;
+                }
+            } else {
+                xs[lr] = x[j];
+                if (lr < R) {
+                    od[lr] = omega * dinv[j];
+                    bs[lr] = (T)b[j];
+                }
+            }
+        }
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar, phase));
+        if (!ok) {
+            if ((threadIdx.x & 31) == 0) atomicExch(rv.err, (int)CFA_TIMEOUT);
+            abort_flag = 1;
+        }
+        __syncthreads();
+        if (abort_flag) return;
+        for (int lr = threadIdx.x; lr < R; lr += kRingThreads) {
+            const T s = ring_row<V, T>(rr, cs, vv, xs, lr);
+            T y;
+            if (OP == RING_JAC) y = xs[lr] + od[lr] * (bs[lr] - s);
+            else y = fma_rn(od[lr], bs[lr] - s, xs[lr]);
+            ys[lr] = y;
+            if (OP != RING_JAC && lr < nr) xout[r0 + lr] = y;
+        }
+        __syncthreads();
+        for (int lr = threadIdx.x; lr < nr; lr += kRingThreads) {
+            const int row = r0 + lr;
+            double bd = 0.0, qd = 0.0;
+            if constexpr (RZ) {
+                bd = (double)b[row];
+                if (rzf.flexible) qd = rzf.q[row];
+            }
+            const T s = ring_row<V, T>(rr, cs, vv, ys, lr);
+            if (OP == RING_JAC) {
+                const O o = (O)(ys[lr] + od[lr] * (bs[lr] - s));
+                out[row] = o;
+                if constexpr (RZ) {
+                    dots[0] += bd * (double)o;
+                    if (rzf.flexible) dots[1] += (double)o * qd;
+                }
+            } else {
+                out[row] = (O)(bs[lr] - s);
+            }
+        }
+        __syncthreads();   // the tile's shared memory is free again
+        phase ^= 1u;
+        first = false;
+    }
+    if constexpr (RZ) {
+        __shared__ double sh[2 * kWarps];
+        block_sum<2>(dots, sh);
+        if (publish_partials<2>(dots, rzf.part, rzf.counter)) {
+            reduce_partials<2>(dots, rzf.part, rzf.counter, sh);
+            if (threadIdx.x == 0) {
+                const double rz_old = *rzf.rz;
+                *rzf.beta = rzf.flexible ? -(*rzf.alpha) * dots[1] / (rz_old + 1.0e-30) : dots[0] / (rz_old + 1.0e-30);
+                *rzf.rz = dots[0];
+            }
+        }
+    }
+}
+
+// Launches (or, dry, only prepares) one pair of sweeps
+template <int OP, class V, class T, class B, class O, bool RZ>
+static void ring_launch(cfa_ctx* ctx, bool dry, const RingTiles& R, int* err, const T* dinv, T omega, const B* b,
+                        const T* x, T* xout, O* out, const int* done, const RzFuse& rz) {
+    const void* kernel = (const void*)k_ring<OP, V, T, B, O, RZ>;
+    const int smem = ring_smem(R, (int)sizeof(V), (int)sizeof(T));
+    if (dry) {
+        static std::once_flag once;
+        std::call_once(once, [&] { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingMaxSmem); });
+        return;
+    }
+    const RingView<V> rv{R.n, R.rows, R.ntiles, R.rp_stride, R.max_rows, R.max_local, R.max_ne, R.meta.p, R.halo.p,
+                         R.rp.p, R.ci.p, ring_values(R, V()), err};
+    const int grid = std::max(1, std::min(R.ntiles, std::max(1, tile_occupancy(kernel, smem)) * ctx->num_sms));
+    CFA_LAUNCH(ctx, (k_ring<OP, V, T, B, O, RZ>), grid, kRingThreads, smem, rv, dinv, omega, b, x, xout, out, done, rz);
+}
+
+template <int OP, class V, class T, class B, class O>
+static void ring_sweeps(cfa_ctx* ctx, bool dry, const RingTiles& R, int* err, const T* dinv, T omega, const B* b,
+                        const T* x, T* xout, O* out, const int* done, const RzFuse* rz = nullptr) {
+    constexpr bool kRz = OP == RING_JAC && std::is_same<O, double>::value && std::is_same<B, double>::value;
+    if (dry || (kRz && rz))
+        ring_launch<OP, V, T, B, O, kRz>(ctx, dry, R, err, dinv, omega, b, x, xout, out, done, rz ? *rz : RzFuse{});
+    if (dry || !(kRz && rz))
+        ring_launch<OP, V, T, B, O, false>(ctx, dry, R, err, dinv, omega, b, x, xout, out, done, RzFuse{});
+}
+
+// ---------------------------------------------------------------------------------------------
 // launch helpers with the TPR dispatch
 // ---------------------------------------------------------------------------------------------
 #define CFA_TPR_SWITCH(tpr, ...)                                                               \
@@ -1439,7 +1615,14 @@ static void vcycle_tiled(cfa_ctx* ctx, cfa_amg* amg, int l, const B* b, double* 
     const T* dinv = TVec<T>::dinv(L);
     T* x = TVec<T>::x(L);
     T* t = TVec<T>::t(L);
-    if (s >= 2 && c0 && !cg) {   // the first iterate formed by the caller
+    const bool ring = L.ring.ok && !cg;   // level 0, two smoothing steps: sweeps in pairs
+    if (ring) {
+        if (c0 || dry)
+            ring_sweeps<RING_PREC, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, c0, x, TVec<T>::r(L), done);
+        if (!c0 || dry)
+            ring_sweeps<RING_PRE, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, (const T*)nullptr, x,
+                                              TVec<T>::r(L), done);
+    } else if (s >= 2 && c0 && !cg) {   // the first iterate formed by the caller
         vct<VC_PREC, V, T, B, T>(ctx, dry, tA, err, dinv, omega, b, c0, x, done);
     } else if (s >= 2) {
         if (dry) vct<VC_PREC, V, T, B, T>(ctx, dry, tA, err, dinv, omega, b, (const T*)nullptr, x, done);
@@ -1451,7 +1634,7 @@ static void vcycle_tiled(cfa_ctx* ctx, cfa_amg* amg, int l, const B* b, double* 
                                                                                     : (const void*)L.A.v.p),
                                            dinv, omega, b, 0, x, done));
     }
-    for (int k = 2; k < s; ++k) {
+    for (int k = 2; k < s && !ring; ++k) {
         vct<VC_JAC, V, T, B, T>(ctx, dry, tA, err, dinv, omega, b, (const T*)x, t, done);
         std::swap(x, t);
     }
@@ -1460,8 +1643,9 @@ static void vcycle_tiled(cfa_ctx* ctx, cfa_amg* amg, int l, const B* b, double* 
     if (L.fusedQ) {   // cb = R b - (R A) x in one pass
         vct<VC_RESTRICT, V, T, B, T>(ctx, dry, tQ, err, dinv, omega, b, (const T*)x, cb, done);
     } else {
-        vct<VC_RES, V, T, B, T>(ctx, dry, tA, err, dinv, omega, b, (const T*)x, TVec<T>::r(L), done, nullptr,
-                                nullptr, cg);
+        if (!ring)
+            vct<VC_RES, V, T, B, T>(ctx, dry, tA, err, dinv, omega, b, (const T*)x, TVec<T>::r(L), done, nullptr,
+                                    nullptr, cg);
         vct<VC_SPMV, V, T, T, T>(ctx, dry, tR, err, dinv, omega, (const T*)nullptr, (const T*)TVec<T>::r(L), cb,
                                  done);
     }
@@ -1490,6 +1674,11 @@ static void vcycle_tiled(cfa_ctx* ctx, cfa_amg* amg, int l, const B* b, double* 
         k0 = 1;
     } else {
         vct<VC_ADD, V, T, T, T>(ctx, dry, tP, err, dinv, omega, (const T*)nullptr, cx, x, done);
+    }
+    if (ring) {
+        ring_sweeps<RING_JAC, V, T, B, double>(ctx, dry, L.ring, err, dinv, omega, b, (const T*)x, (T*)nullptr, z, done,
+                                               rz);
+        return;
     }
     for (int k = k0; k < s; ++k) {
         if (l == 0 && k == s - 1) {
@@ -1539,10 +1728,12 @@ bool amg_prescale(const cfa_amg* amg, PreScale* out, bool fp64) {
 // Off unless CFA_CG_FUSE_UPDATE=1: measured on the 402k-vertex step the folded form was not
 // faster (13.78 against 13.60 ms without setup): the pre-smoothing pass gathers q beside r for every entry and the
 // residual pass takes the grid reduction, which cost what the update kernel's launch saved.
-bool amg_can_fuse_update(const cfa_amg* amg) {
+static bool cg_update_fused() {
     const char* e = std::getenv("CFA_CG_FUSE_UPDATE");
-    const bool on = e && e[0] == '1';
-    return on && amg && !amg->levels.empty() && amg->tiled && amg->opts.smooth_steps == 2 &&
+    return e && e[0] == '1';
+}
+bool amg_can_fuse_update(const cfa_amg* amg) {
+    return cg_update_fused() && amg && !(!amg->levels.empty() && amg->levels[0].ring.ok) && !amg->levels.empty() && amg->tiled && amg->opts.smooth_steps == 2 &&
            !amg->levels[0].fusedQ;
 }
 
@@ -2433,7 +2624,12 @@ static cfa_status prepare_level(cfa_ctx* ctx, cfa_amg* amg, AmgLevel& L) {
         return level_vectors64(ctx, L, L.A.rows);
     }
     if (fuse_level(amg, L)) CFA_PROPAGATE(build_fused(ctx, amg, L, vb, fuse_prolongation(amg, L)));
+    L.ring.ok = false;
+    if (l == 0 && o.smooth_steps == 2 && !L.fusedQ && !L.fusedW && !cg_update_fused())
+        CFA_PROPAGATE(build_ring(ctx, L.A.rows, L.A.nnz, L.A.rp.p, L.A.ci.p, L.A.v.p, vb == 4,
+                                 vb == 8 || amg->phase_switch > 0.0, L.ring));
     for (DCsr* M : {&L.A, &L.P, &L.R}) {
+        if (M == &L.A && L.ring.ok) continue;
         TiledCsr& T = M == &L.A ? L.tA : M == &L.P ? L.tP : L.tR;
         HostBuf<int>& hr = amg->scratch.h_rp;
         CFA_CUDA(hr.ensure(M->rows + 1));

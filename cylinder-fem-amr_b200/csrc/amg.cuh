@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "ring.cuh"
 #include "tiled.cuh"
 
 namespace cfa {
@@ -27,6 +28,7 @@ struct AmgLevel {
     // FP64 copies of tA, tP, tR, tQ, tW in a mixed-precision hierarchy, for the FP64 V-cycles that
     // a solve runs first (amg_fp64_phase); empty otherwise
     TiledCsr tA64, tP64, tR64, tQ64, tW64;
+    RingTiles ring;                // level 0: two sweeps per pass (ring.cuh), in place of tA
     bool fusedQ = false, fusedW = false;
     bool ra_spgemm = false;        // R A formed by SpGEMM (A not symmetric) rather than as (A P)^T
     DCsr AP;                       // A P of the Galerkin product (rows 0 after a remap changed P)

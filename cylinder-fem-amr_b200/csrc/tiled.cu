@@ -207,7 +207,7 @@ void allow_tile_kernel(const void* kernel) {
 
 // Resident blocks per SM of a tile kernel with this much dynamic shared memory, as the runtime
 // computes it from the kernel's registers too (cached; 0 when the query fails).
-static int tile_occupancy(const void* kernel, int smem) {
+int tile_occupancy(const void* kernel, int smem) {
     static std::mutex mu;
     static std::unordered_map<std::string, int> cache;
     char key[64];

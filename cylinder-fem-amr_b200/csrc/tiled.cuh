@@ -330,6 +330,8 @@ struct TileLaunch {
     int grid = 1, smem = 0, tpr = 1;
 };
 TileLaunch tile_launch(const cfa_ctx* ctx, const TiledCsr& T, const void* kernel);
+// Resident blocks per SM of a kernel of kTileThreads threads with this much dynamic shared memory.
+int tile_occupancy(const void* kernel, int smem);
 // Raises the kernel's dynamic shared memory limit to kTileStages tiles of the budget (once per kernel;
 // call outside stream capture).
 void allow_tile_kernel(const void* kernel);
