@@ -455,6 +455,18 @@ k_opt_k(TileView tv, const int* __restrict__ tag, OutletBc bc, const double* __r
     }
 }
 
+// p = z + beta p on its own, for the systems whose operator then gathers one vector (split_p).
+// HBM-bound, 24 bytes a row (4.2M vertices: 16 us).
+__global__ void __launch_bounds__(kThreads)
+k_cg_p(int n, const double* __restrict__ z, const double* __restrict__ beta_ptr, double* __restrict__ p,
+       const int* __restrict__ done) {
+    CFA_GRID_DEP();
+    if (*done) return;
+    const double beta = *beta_ptr;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        p[i] = __fma_rn(beta, p[i], z[i]);
+}
+
 // ||b|| (solve_pcg :205-209)
 __global__ void __launch_bounds__(kThreads)
 k_cg_bnorm(int n, const double* __restrict__ b, CgState* __restrict__ st, double* __restrict__ part,
@@ -563,7 +575,7 @@ k_cg_update(int n, double* __restrict__ x, double* __restrict__ r, const double*
         x[i] += alpha * pi;
         const double ri = r[i] + -alpha * q[i];
         r[i] = ri;
-        p[i] = pi;
+        if (p) p[i] = pi;
         if (c0) c0[i] = SC(omega0 * dinv0[i]) * (SC)ri;   // the level-0 pre-smoothing's (omega D^-1) b, rounded
         v[0] += ri * ri;
         if (JAC) {
@@ -1506,6 +1518,17 @@ static int pcg_flexible(const cfa_amg* amg) {
     return (e && e[0] == '0') ? 0 : 1;
 }
 
+// Whether p = z + beta p is a kernel of its own (k_cg_p) ahead of a one-pass operator, instead of
+// being formed for every entry the operator gathers. The operator then gathers one vector in place
+// of two and writes none, and p updated in place needs no copy by the CG's update: the same bytes, half
+// the gathers, one launch more. CG solve, formed in the operator against split: 69k vertices 3.46 -> 3.45
+// ms, 141k 5.05 -> 4.90, 402k 8.87 -> 8.57, 651k 11.39 -> 10.82, 4.2M 88.5 -> 83.0 ms, but 8k 2.09 -> 2.12 ms.
+// The line is the rings' (two tiles of 256 rows per SM): above it launches no longer show.
+static bool split_p(const cfa_ctx* ctx, const PcgWork& W, const PcgArgs& a) {
+    return W.tiled && (!a.oss || W.fused) && a.amg && !a.host_ops() && !amg_can_fuse_update(a.amg) &&
+           (long long)a.n > 512LL * ctx->num_sms;
+}
+
 static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piece, CondArg cond) {
     const int n = a.n;
     const int gv = row_grid(ctx, n, 1);
@@ -1513,7 +1536,12 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
     const int* done = &st->done;
     if (piece == 0) {
         // q = A pn with pn = z + beta p
-        CFA_PROPAGATE(pcg_operator(ctx, W, a, W.z.p, W.p.p, &st->beta, W.pn.p, W.q.p, !a.extra, cond, done));
+        if (split_p(ctx, W, a)) {
+            CFA_LAUNCH(ctx, k_cg_p, gv, kThreads, 0, n, (const double*)W.z.p, (const double*)&st->beta, W.p.p, done);
+            CFA_PROPAGATE(pcg_operator(ctx, W, a, W.p.p, W.p.p, nullptr, nullptr, W.q.p, true, cond, done));
+        } else {
+            CFA_PROPAGATE(pcg_operator(ctx, W, a, W.z.p, W.p.p, &st->beta, W.pn.p, W.q.p, !a.extra, cond, done));
+        }
     } else if (piece == 1) {
         if (a.extra)
             CFA_LAUNCH(ctx, k_cg_pq, gv, kThreads, 0, n, (const double*)W.pn.p, (const double*)W.q.p, st, W.part.p,
@@ -1524,18 +1552,22 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
             // pre-smoothing's scaled residual where the V-cycle takes it
             const bool fuse_update = !a.prec && amg_can_fuse_update(a.amg);
             PreScale ps{};
+            // the direction, and where it is copied to unless it was updated in place
+            const bool split = split_p(ctx, W, a);
+            const double* dir = split ? W.p.p : W.pn.p;
+            double* keep = split ? nullptr : W.p.p;
             const bool prescale = !a.prec && !fuse_update && amg_prescale(a.amg, &ps, a.vc64 != 0);
             if (!fuse_update) {
                 if (prescale && ps.fp32)
-                    CFA_LAUNCH(ctx, (k_cg_update<false, float>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p, W.q.p,
+                    CFA_LAUNCH(ctx, (k_cg_update<false, float>), gv, kThreads, 0, n, W.x.p, W.r.p, dir, keep, W.q.p,
                                (const double*)nullptr, (double*)nullptr, st, W.part.p, W.counter.p, cond,
                                (const float*)ps.dinv, (float)ps.omega, reinterpret_cast<float*>(W.c0.p));
                 else if (prescale)
-                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p,
+                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, W.x.p, W.r.p, dir, keep,
                                W.q.p, (const double*)nullptr, (double*)nullptr, st, W.part.p, W.counter.p, cond,
                                (const double*)ps.dinv, ps.omega, W.c0.p);
                 else
-                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, W.x.p, W.r.p, W.pn.p, W.p.p,
+                    CFA_LAUNCH(ctx, (k_cg_update<false, double>), gv, kThreads, 0, n, W.x.p, W.r.p, dir, keep,
                                W.q.p, (const double*)nullptr, (double*)nullptr, st, W.part.p, W.counter.p, cond,
                                (const double*)nullptr, 0.0, (double*)nullptr);
             }
