@@ -71,15 +71,15 @@ struct HostBuf {
 
 // Setup temporaries, kept across setups (grow-only): no allocation in a repeated setup.
 struct SetupScratch {
-    DevBuf<int> sg_ub, sg_cnt, sg_scol, sg_big, tr_keys, tr_idx, tr_perm, tr_row_of, cnt, p0rp, ierr;
-    DevBuf<long long> sg_off;
+    DevBuf<int> sg_cnt, sg_scol, sg_mid, sg_big, tr_keys, tr_idx, tr_perm, tr_row_of, cnt, p0rp, ierr;
+    DevBuf<long long> sg_ub, sg_off;
     DevBuf<double> sg_sval, pow_x, pow_y, pow_py, pow_px, pow_st, p0v, M, colbuf;
     DevBuf<unsigned char> strong;
     DevBuf<int> ag_trp, ag_tci, ag_fill, ag_rank, ag_agg1, ag_agg2, ag_size, ag_flag, ag_cptr, ag_conf;   // device aggregation
     DevBuf<unsigned char> ag_state;
     HostBuf<int> h_ag;                  // flag / totals read back by the aggregation rounds
     DevBuf<char> cub_tmp;
-    HostBuf<int> h_rp, h_ci, h_cnt, h_ub, h_agg, h_p0rp;
+    HostBuf<int> h_rp, h_ci, h_cnt, h_agg, h_p0rp;
     HostBuf<long long> h_off;
     HostBuf<unsigned char> h_strong;
     HostBuf<double> h_p0v, h_st;
