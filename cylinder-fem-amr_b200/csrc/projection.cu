@@ -5,6 +5,8 @@
 // The reference scatters element contributions with FP64 atomics (an order that changes run to
 // run). Here every node gathers its elements through the mesh's incidence list (ascending element
 // order), and the forces are summed by a fixed-order two-stage reduction: deterministic results.
+#include <mutex>
+
 #include "internal.cuh"
 #include "mesh.cuh"
 
@@ -68,6 +70,92 @@ k_node_gradients(int n, const int* __restrict__ ev, const double* __restrict__ x
     if (stiff) stiff[i] += s;
     if (gdx) { gdx[i] = sx; gdy[i] = sy; }
     if (vort_num) vort_num[i] = sw;
+}
+
+// k_node_gradients on element tiles (elemtile.cuh): the element's six values once, then the nodes.
+// Bound by latency (elemtile.cuh): 27.9 -> 17.3 us at 120k vertices; the recovered gradient 23.1 -> 15.5 us.
+__global__ void __launch_bounds__(kEtThreads)
+k_node_gradients_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
+                       const double* __restrict__ y, const double* __restrict__ f, double c,
+                       double* __restrict__ stiff, const double* __restrict__ dp, const double* __restrict__ u,
+                       const double* __restrict__ v, double* __restrict__ gdx, double* __restrict__ gdy,
+                       double* __restrict__ vort_num) {
+    extern __shared__ __align__(16) double et_rec[];   // [8][tv.stride]: stiffness by vertex (3) and its
+    // factor, grad dp (2), vorticity, area / 3; the factors enter by fused multiply-adds as in the gather
+    const EtBlock b = et_block(tv, n);
+    const int S = tv.stride;
+    CFA_GRID_DEP();
+    for (int le = threadIdx.x; le < b.ne; le += kEtThreads) {
+        const int e = tv.elems[b.i0 + le];
+        const int nd[3] = {ev[3 * e], ev[3 * e + 1], ev[3 * e + 2]};
+        const ElemGrad g = elem_grad(nd, x, y);
+        double* rec = et_rec + le;
+        if (!g.ok) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) rec[q * S] = 0.0;
+            continue;
+        }
+        if (stiff) {
+            const double gx = f[nd[0]] * g.dNdx[0] + f[nd[1]] * g.dNdx[1] + f[nd[2]] * g.dNdx[2];
+            const double gy = f[nd[0]] * g.dNdy[0] + f[nd[1]] * g.dNdy[1] + f[nd[2]] * g.dNdy[2];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) rec[a * S] = g.dNdx[a] * gx + g.dNdy[a] * gy;
+            rec[3 * S] = c * g.area;
+        }
+        rec[7 * S] = g.area / 3.0;
+        if (gdx) {
+            rec[4 * S] = dp[nd[0]] * g.dNdx[0] + dp[nd[1]] * g.dNdx[1] + dp[nd[2]] * g.dNdx[2];
+            rec[5 * S] = dp[nd[0]] * g.dNdy[0] + dp[nd[1]] * g.dNdy[1] + dp[nd[2]] * g.dNdy[2];
+        }
+        if (vort_num) {
+            const double dvdx = v[nd[0]] * g.dNdx[0] + v[nd[1]] * g.dNdx[1] + v[nd[2]] * g.dNdx[2];
+            const double dudy = u[nd[0]] * g.dNdy[0] + u[nd[1]] * g.dNdy[1] + u[nd[2]] * g.dNdy[2];
+            rec[6 * S] = dvdx - dudy;
+        }
+    }
+    __syncthreads();
+    for (int i = b.r0 + threadIdx.x; i < b.r1; i += kEtThreads) {
+        double s = 0.0, sx = 0.0, sy = 0.0, sw = 0.0;
+        for (int k = tv.inc_ptr[i]; k < tv.inc_ptr[i + 1]; ++k) {
+            const int q = tv.rcode[k], le = q >> 2;
+            const double w = et_rec[7 * S + le];
+            if (stiff) s = __fma_rn(et_rec[3 * S + le], et_rec[(q & 3) * S + le], s);
+            if (gdx) {
+                sx = __fma_rn(w, et_rec[4 * S + le], sx);
+                sy = __fma_rn(w, et_rec[5 * S + le], sy);
+            }
+            if (vort_num) sw = __fma_rn(w, et_rec[6 * S + le], sw);
+        }
+        if (stiff) stiff[i] += s;
+        if (gdx) { gdx[i] = sx; gdy[i] = sy; }
+        if (vort_num) vort_num[i] = sw;
+    }
+}
+
+__global__ void k_recovered_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev,
+                                           const double* __restrict__ x, const double* __restrict__ y,
+                                           const double* __restrict__ u, const double* __restrict__ v, double u_max,
+                                           double H, double* __restrict__ grad_rec);
+static void allow_post_kernels() {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaFuncSetAttribute(k_node_gradients_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, kEtMaxSmem);
+        cudaFuncSetAttribute(k_recovered_gradient_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, kEtMaxSmem);
+    });
+}
+
+static cfa_status node_gradients(cfa_ctx* ctx, const cfa_mesh* m, const double* f, double c, double* stiff,
+                                 const double* dp, const double* u, const double* v, double* gdx, double* gdy,
+                                 double* vort_num) {
+    allow_post_kernels();
+    if (m->et.ok)
+        CFA_LAUNCH(ctx, k_node_gradients_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 8), m->tiles(), m->n, m->ev, m->x,
+                   m->y, f, c, stiff, dp, u, v, gdx, gdy, vort_num);
+    else
+        CFA_LAUNCH(ctx, k_node_gradients, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y, m->inc_ptr.p,
+                   m->inc.p, f, c, stiff, dp, u, v, gdx, gdy, vort_num);
+    CFA_CHECK_LAUNCH();
+    return CFA_OK;
 }
 
 // k_velocity_pressure_correction (fem_kernels.cuh:585-610):
@@ -182,6 +270,50 @@ k_recovered_gradient(int n, const int* __restrict__ ev, const double* __restrict
     for (int c = 0; c < 4; ++c) grad_rec[(size_t)c * n + i] = s[c];
 }
 
+// k_recovered_gradient on element tiles
+__global__ void __launch_bounds__(kEtThreads)
+k_recovered_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
+                           const double* __restrict__ y, const double* __restrict__ u, const double* __restrict__ v,
+                           double u_max, double H, double* __restrict__ grad_rec) {
+    extern __shared__ __align__(16) double et_rec[];   // [5][tv.stride]
+    const EtBlock b = et_block(tv, n);
+    const int S = tv.stride;
+    CFA_GRID_DEP();
+    for (int le = threadIdx.x; le < b.ne; le += kEtThreads) {
+        const int e = tv.elems[b.i0 + le];
+        const int nd[3] = {ev[3 * e], ev[3 * e + 1], ev[3 * e + 2]};
+        const ElemGrad g = elem_grad(nd, x, y);
+        double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (g.ok) {
+            double ud[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const double ya = y[nd[a]];
+                ud[a] = u[nd[a]] - 4.0 * u_max * ya * (H - ya) / (H * H);
+            }
+            r[0] = ud[0] * g.dNdx[0] + ud[1] * g.dNdx[1] + ud[2] * g.dNdx[2];
+            r[1] = ud[0] * g.dNdy[0] + ud[1] * g.dNdy[1] + ud[2] * g.dNdy[2];
+            r[2] = v[nd[0]] * g.dNdx[0] + v[nd[1]] * g.dNdx[1] + v[nd[2]] * g.dNdx[2];
+            r[3] = v[nd[0]] * g.dNdy[0] + v[nd[1]] * g.dNdy[1] + v[nd[2]] * g.dNdy[2];
+            r[4] = g.area / 3.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q) et_rec[q * S + le] = r[q];
+    }
+    __syncthreads();
+    for (int i = b.r0 + threadIdx.x; i < b.r1; i += kEtThreads) {
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int k = tv.inc_ptr[i]; k < tv.inc_ptr[i + 1]; ++k) {
+            const int le = tv.rcode[k] >> 2;
+            const double w = et_rec[4 * S + le];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s[q] = __fma_rn(w, et_rec[q * S + le], s[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) grad_rec[(size_t)q * n + i] = s[q];
+    }
+}
+
 // k_compute_amr_error_indicator (fem_kernels.cuh:995-1035): per element the disturbance
 // vorticity times h_K and the P1 interpolation-error estimate from the recovered gradient.
 __global__ void k_amr_indicator(int ne, int n, const int* __restrict__ ev, const double* __restrict__ x,
@@ -220,21 +352,14 @@ extern "C" {
 cfa_status cfa_stiffness_apply(cfa_ctx* ctx, const cfa_mesh* m, const double* f, double c, double* out) {
     CFA_ENTER(ctx);
     CFA_ARG(m && f && out);
-    CFA_LAUNCH(ctx, k_node_gradients, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y, m->inc_ptr.p,
-               m->inc.p, f, c, out, (const double*)nullptr, (const double*)nullptr, (const double*)nullptr,
-               (double*)nullptr, (double*)nullptr, (double*)nullptr);
-    CFA_CHECK_LAUNCH();
-    return CFA_OK;
+    return node_gradients(ctx, m, f, c, out, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
 }
 
 cfa_status cfa_grad_dp_vorticity(cfa_ctx* ctx, const cfa_mesh* m, const double* dp, const double* u,
                                  const double* v, double* grad_dp_x, double* grad_dp_y, double* vort_num) {
     CFA_ENTER(ctx);
     CFA_ARG(m && dp && u && v && grad_dp_x && grad_dp_y && vort_num);
-    CFA_LAUNCH(ctx, k_node_gradients, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y, m->inc_ptr.p,
-               m->inc.p, (const double*)nullptr, 0.0, (double*)nullptr, dp, u, v, grad_dp_x, grad_dp_y, vort_num);
-    CFA_CHECK_LAUNCH();
-    return CFA_OK;
+    return node_gradients(ctx, m, nullptr, 0.0, nullptr, dp, u, v, grad_dp_x, grad_dp_y, vort_num);
 }
 
 cfa_status cfa_velocity_pressure_correction(cfa_ctx* ctx, const cfa_mesh* m, double dt, double rho, double p_update,
@@ -257,9 +382,8 @@ cfa_status cfa_project_step(cfa_ctx* ctx, const cfa_mesh* m, double dt_proj, dou
     CFA_ENTER(ctx);
     CFA_ARG(m && mass_lumped && dp && div_num && grad_dp_x && grad_dp_y && vort_num && u && v && p);
     if (rotational_from_dp) CFA_CUDA(cudaMemsetAsync(div_num, 0, (size_t)m->n * sizeof(double), ctx->stream));
-    CFA_LAUNCH(ctx, k_node_gradients, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y, m->inc_ptr.p,
-               m->inc.p, (const double*)dp, -dt_proj / rho, rotational_from_dp ? div_num : (double*)nullptr, dp,
-               (const double*)u, (const double*)v, grad_dp_x, grad_dp_y, vort_num);
+    CFA_PROPAGATE(node_gradients(ctx, m, dp, -dt_proj / rho, rotational_from_dp ? div_num : nullptr, dp, u, v,
+                                 grad_dp_x, grad_dp_y, vort_num));
     CFA_LAUNCH(ctx, k_correction, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->tag, m->bc, dt_proj, rho, 1.0,
                rot_coeff, (const double*)div_num, mass_lumped, (const double*)grad_dp_x, (const double*)grad_dp_y,
                (const double*)vort_num, dp, u, v, p, vort);
@@ -284,8 +408,13 @@ cfa_status cfa_recovered_gradient(cfa_ctx* ctx, const cfa_mesh* m, const double*
                                   double H, double* grad_rec) {
     CFA_ENTER(ctx);
     CFA_ARG(m && u && v && grad_rec && H > 0.0);
-    CFA_LAUNCH(ctx, k_recovered_gradient, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y,
-               m->inc_ptr.p, m->inc.p, u, v, u_max, H, grad_rec);
+    allow_post_kernels();
+    if (m->et.ok)
+        CFA_LAUNCH(ctx, k_recovered_gradient_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 5), m->tiles(), m->n, m->ev,
+                   m->x, m->y, u, v, u_max, H, grad_rec);
+    else
+        CFA_LAUNCH(ctx, k_recovered_gradient, ceil_div(m->n, kThreads), kThreads, 0, m->n, m->ev, m->x, m->y,
+                   m->inc_ptr.p, m->inc.p, u, v, u_max, H, grad_rec);
     CFA_CHECK_LAUNCH();
     return CFA_OK;
 }

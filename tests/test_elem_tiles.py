@@ -109,3 +109,51 @@ def test_assembly_matches_the_oracle(name, outlet_dirichlet):
     cfa.apply_bc_pressure(ctx, dm, K, rhs, dp1, t(omass))
     for a, b in ((K, K2), (rhs, rhs2), (div, div2), (dp1, dp2), (oss, oss2), (im, im2)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_node_gradients_match_the_formulas(name):
+    import torch
+    import cfa_b200 as cfa
+    from oracle import oracle as O
+    m = CASES[name]()
+    ctx = cfa.default_context()
+    rp, ci = O.csr_build(m.n, m.elem_v)
+    dm = cfa.DeviceMesh(ctx, m, torch.from_numpy(rp).to("cuda"), torch.from_numpy(ci).to("cuda"))
+    n, t = m.n, m.tri.astype(np.int64)
+    X, Y = m.x[t], m.y[t]
+    area = 0.5 * np.abs((X[:, 1] - X[:, 0]) * (Y[:, 2] - Y[:, 0]) - (X[:, 2] - X[:, 0]) * (Y[:, 1] - Y[:, 0]))
+    gx = np.stack([Y[:, 1] - Y[:, 2], Y[:, 2] - Y[:, 0], Y[:, 0] - Y[:, 1]], 1) / (2 * area)[:, None]
+    gy = np.stack([X[:, 2] - X[:, 1], X[:, 0] - X[:, 2], X[:, 1] - X[:, 0]], 1) / (2 * area)[:, None]
+
+    def nodes(e):          # e: one value per element, or per element and vertex
+        out, size = np.zeros(n), np.zeros(n)
+        e = np.broadcast_to(e if e.ndim == 2 else e[:, None], t.shape)
+        np.add.at(out, t.ravel(), e.ravel())
+        np.add.at(size, t.ravel(), np.abs(e).ravel())
+        return out, size.max()
+
+    grad = lambda f: ((f[t] * gx).sum(1), (f[t] * gy).sum(1))
+    u, v, dp = (F.fourier_field(m.x, m.y, k) for k in (1, 2, 3))
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float64)).to("cuda")
+    z = lambda k: torch.full((k,), float("nan"), dtype=torch.float64, device="cuda")
+
+    def close(got, want):  # sums of at most 3100 terms, each a few dozen roundings
+        assert np.abs(got.cpu().numpy() - want[0]).max() <= 1e-12 * want[1]
+
+    w = area / 3
+    (dx, dy), curl = grad(dp), grad(v)[0] - grad(u)[1]
+    a, b, c = z(n), z(n), z(n)
+    cfa.grad_dp_vorticity(ctx, dm, d(dp), d(u), d(v), a, b, c)
+    for got, e in ((a, w * dx), (b, w * dy), (c, w * curl)):
+        close(got, nodes(e))
+    s0 = np.linspace(-1, 1, n)
+    s = d(s0)
+    cfa.stiffness_apply(ctx, dm, d(dp), -0.37, s)
+    want, size = nodes(-0.37 * area[:, None] * (gx * dx[:, None] + gy * dy[:, None]))
+    close(s, (want + s0, max(size, 1.0)))
+    mass, rec, err = d(nodes(w)[0]), z(4 * n), z(2 * m.ne)
+    cfa.amr_indicators(ctx, dm, d(u), d(v), 1.5, 1.0, mass, rec, err)
+    ud = u - 6.0 * m.y * (1 - m.y)
+    for k, e in enumerate((*grad(ud), *grad(v))):
+        close(rec[k * n:(k + 1) * n], nodes(w * e))
