@@ -968,6 +968,24 @@ __device__ __forceinline__ double fma_rn(double a, double b, double c) { return 
 enum VcOp { VC_PRE = 0, VC_JAC = 1, VC_RES = 2, VC_SPMV = 3, VC_ADD = 4, VC_RESTRICT = 5, VC_ADDJAC = 6, VC_PREC = 7 };
 constexpr int kSecondVec = (int)0x80000000u;
 
+// |r| and the stopping test of the CG's update kernel (solve_pcg, src/cfa/linalg.cuh:239-246), one thread
+__device__ __forceinline__ void cg_stop_test(CgState* st, double rr, CondArg cond) {
+    const double rnorm = sqrt(rr);
+    st->rel = rnorm / st->bnorm;
+    const int it = st->iter + 1;
+    st->iter = it;
+    if (rnorm < st->tol * st->bnorm) {
+        st->done = 1;
+        st->converged = 1;
+        set_cond(cond, 0);
+    } else if (it >= st->max_iter) {
+        st->done = 1;
+        st->converged = 0;
+        st->status = CFA_NOT_CONVERGED;
+        set_cond(cond, 0);
+    }
+}
+
 template <int TPR, int OP, class V, class T, class B, class O, bool RZ = false, bool CGU = false>
 __global__ void __launch_bounds__(kTileThreads)
 k_vct(TileView tv, const T* __restrict__ dinv, T omega, const B* __restrict__ b, const T* __restrict__ x,
@@ -1084,28 +1102,11 @@ k_vct(TileView tv, const T* __restrict__ dinv, T omega, const B* __restrict__ b,
     });
     if (!go) return;
     if constexpr (CGU && OP == VC_RES) {
-        // |r| and the stopping test of the CG's update kernel (solve_pcg, src/cfa/linalg.cuh:239-246)
         __shared__ double sh[2 * kWarps];
         block_sum<2>(dots, sh);
         if (publish_partials<2>(dots, cgf.part, cgf.counter)) {
             reduce_partials<2>(dots, cgf.part, cgf.counter, sh);
-            if (threadIdx.x == 0) {
-                CgState* st = cgf.st;
-                const double rnorm = sqrt(dots[0]);
-                st->rel = rnorm / st->bnorm;
-                const int it = st->iter + 1;
-                st->iter = it;
-                if (rnorm < st->tol * st->bnorm) {
-                    st->done = 1;
-                    st->converged = 1;
-                    set_cond(cgf.cond, 0);
-                } else if (it >= st->max_iter) {
-                    st->done = 1;
-                    st->converged = 0;
-                    st->status = CFA_NOT_CONVERGED;
-                    set_cond(cgf.cond, 0);
-                }
-            }
+            if (threadIdx.x == 0) cg_stop_test(cgf.st, dots[0], cgf.cond);
         }
     }
     if constexpr (RZ) {
@@ -1167,10 +1168,12 @@ static void vct(cfa_ctx* ctx, bool dry, const TiledCsr& M, int* err, const T* di
 // ---------------------------------------------------------------------------------------------
 // RING_PRE: x = VC_PRE of b, out = b - A x; RING_PREC: the same with the first iterate c = x given;
 // RING_JAC: out = two Jacobi sweeps from x (RZ: with the CG's dots of out). xout: RING_PRE(C)'s x.
+// RING_CGU: RING_PRE of the residual r - alpha q after the CG's update, which it also does on its own
+// rows (k_cg_update's operations), with |r| and the stopping test.
 // Bound by latency at the sizes that take it (ring_rows, ring.cu): one round of gathers, then two
 // sweeps from shared memory, in place of two kernels. 8k vertices: a pair of kernels 7.4 us -> 4.1 us,
 // the FP64 V-cycle 28.7 -> 21.0 us; 37k: 35.2 -> 31.7 us.
-enum RingOp { RING_PRE = 0, RING_PREC = 1, RING_JAC = 2 };
+enum RingOp { RING_PRE = 0, RING_PREC = 1, RING_JAC = 2, RING_CGU = 3 };
 
 // One row's sum over its entries in order, the loads of a batch ahead of its sums
 template <class V, class T>
@@ -1195,8 +1198,8 @@ __device__ __forceinline__ T ring_row(const unsigned short* rr, const unsigned s
 
 template <int OP, class V, class T, class B, class O, bool RZ>
 __global__ void __launch_bounds__(kRingThreads)
-k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* __restrict__ b, const T* __restrict__ x,
-       T* __restrict__ xout, O* __restrict__ out, const int* __restrict__ done, RzFuse rzf) {
+k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* b, const T* __restrict__ x,
+       T* __restrict__ xout, O* __restrict__ out, const int* __restrict__ done, RzFuse rzf, CgFuse cgf) {
     extern __shared__ __align__(128) unsigned char rsmem[];
     __shared__ uint64_t bar;
     __shared__ int abort_flag;
@@ -1212,6 +1215,8 @@ k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* __restrict_
     double dots[2] = {0.0, 0.0};
     unsigned phase = 0u;
     bool first = true;
+    double alpha = 0.0;
+    double* r_new = nullptr;
     for (int t = blockIdx.x; t < rv.ntiles; t += gridDim.x) {
         const RingMeta m = rv.meta[t];
         const int r0 = t * rv.rows, nr = min(rv.rows, rv.n - r0), R = nr + m.h1, N = R + m.h2;
@@ -1241,9 +1246,35 @@ k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* __restrict_
             if (threadIdx.x == 0) mbar_wait(&bar, 0u);
             return;
         }
+        if constexpr (std::is_same<B, double>::value) {
+            if (first && OP == RING_CGU) {
+                // the buffers of this iteration; its count rises when the last block has finished
+                const bool odd = cgf.st->iter & 1;
+                alpha = cgf.st->alpha;
+                b = odd ? cgf.r_alt : cgf.r;
+                r_new = odd ? cgf.r : cgf.r_alt;
+            } else if (first && rzf.iter && (*rzf.iter & 1)) {
+                b = rzf.r_alt;
+            }
+        }
         for (int lr = threadIdx.x; lr < N; lr += kRingThreads) {
             const int j = lr < nr ? r0 + lr : hl[lr - nr];
-            if (OP == RING_PRE) {
+            if (OP == RING_CGU) {
+                const double rn = (double)b[j] + -alpha * cgf.q[j];
+                const T o = omega * dinv[j], bj = (T)rn;
+                xs[lr] = mul_rn(o, bj);
+                if (lr < R) {
+                    od[lr] = o;
+                    bs[lr] = bj;
+                }
+                if (lr < nr) {   // the CG's update of this row (k_cg_update)
+                    const double pi = cgf.pn[j];
+                    cgf.x[j] += alpha * pi;
+                    r_new[j] = rn;
+                    cgf.p[j] = pi;
+                    dots[0] += rn * rn;
+                }
+            } else if (OP == RING_PRE) {
                 const T o = omega * dinv[j], bj = (T)b[j];
                 xs[lr] = mul_rn(o, bj);
                 if (lr < R) {
@@ -1297,6 +1328,14 @@ k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* __restrict_
         phase ^= 1u;
         first = false;
     }
+    if constexpr (OP == RING_CGU) {
+        __shared__ double sh[2 * kWarps];
+        block_sum<2>(dots, sh);
+        if (publish_partials<2>(dots, cgf.part, cgf.counter)) {
+            reduce_partials<2>(dots, cgf.part, cgf.counter, sh);
+            if (threadIdx.x == 0) cg_stop_test(cgf.st, dots[0], cgf.cond);
+        }
+    }
     if constexpr (RZ) {
         __shared__ double sh[2 * kWarps];
         block_sum<2>(dots, sh);
@@ -1314,7 +1353,7 @@ k_ring(RingView<V> rv, const T* __restrict__ dinv, T omega, const B* __restrict_
 // Launches (or, dry, only prepares) one pair of sweeps
 template <int OP, class V, class T, class B, class O, bool RZ>
 static void ring_launch(cfa_ctx* ctx, bool dry, const RingTiles& R, int* err, const T* dinv, T omega, const B* b,
-                        const T* x, T* xout, O* out, const int* done, const RzFuse& rz) {
+                        const T* x, T* xout, O* out, const int* done, const RzFuse& rz, const CgFuse& cg) {
     const void* kernel = (const void*)k_ring<OP, V, T, B, O, RZ>;
     const int smem = ring_smem(R, (int)sizeof(V), (int)sizeof(T));
     if (dry) {
@@ -1325,17 +1364,20 @@ static void ring_launch(cfa_ctx* ctx, bool dry, const RingTiles& R, int* err, co
     const RingView<V> rv{R.n, R.rows, R.ntiles, R.rp_stride, R.max_rows, R.max_local, R.max_ne, R.meta.p, R.halo.p,
                          R.rp.p, R.ci.p, ring_values(R, V()), err};
     const int grid = std::max(1, std::min(R.ntiles, std::max(1, tile_occupancy(kernel, smem)) * ctx->num_sms));
-    CFA_LAUNCH(ctx, (k_ring<OP, V, T, B, O, RZ>), grid, kRingThreads, smem, rv, dinv, omega, b, x, xout, out, done, rz);
+    CFA_LAUNCH(ctx, (k_ring<OP, V, T, B, O, RZ>), grid, kRingThreads, smem, rv, dinv, omega, b, x, xout, out, done, rz,
+               cg);
 }
 
 template <int OP, class V, class T, class B, class O>
 static void ring_sweeps(cfa_ctx* ctx, bool dry, const RingTiles& R, int* err, const T* dinv, T omega, const B* b,
-                        const T* x, T* xout, O* out, const int* done, const RzFuse* rz = nullptr) {
+                        const T* x, T* xout, O* out, const int* done, const RzFuse* rz = nullptr,
+                        const CgFuse* cg = nullptr) {
     constexpr bool kRz = OP == RING_JAC && std::is_same<O, double>::value && std::is_same<B, double>::value;
-    if (dry || (kRz && rz))
-        ring_launch<OP, V, T, B, O, kRz>(ctx, dry, R, err, dinv, omega, b, x, xout, out, done, rz ? *rz : RzFuse{});
+    const RzFuse f = rz ? *rz : RzFuse{};
+    const CgFuse g = cg ? *cg : CgFuse{};
+    if (dry || (kRz && rz)) ring_launch<OP, V, T, B, O, kRz>(ctx, dry, R, err, dinv, omega, b, x, xout, out, done, f, g);
     if (dry || !(kRz && rz))
-        ring_launch<OP, V, T, B, O, false>(ctx, dry, R, err, dinv, omega, b, x, xout, out, done, RzFuse{});
+        ring_launch<OP, V, T, B, O, false>(ctx, dry, R, err, dinv, omega, b, x, xout, out, done, f, g);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1702,13 +1744,16 @@ static void vcycle_tiled(cfa_ctx* ctx, cfa_amg* amg, int l, const B* b, double* 
     const T* dinv = TVec<T>::dinv(L);
     T* x = TVec<T>::x(L);
     T* t = TVec<T>::t(L);
-    const bool ring = L.ring.ok && !cg;   // level 0, two smoothing steps: sweeps in pairs
+    const bool ring = L.ring.ok;   // level 0, two smoothing steps: sweeps in pairs
     if (ring) {
-        if (c0 || dry)
-            ring_sweeps<RING_PREC, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, c0, x, TVec<T>::r(L), done);
-        if (!c0 || dry)
+        if ((c0 && !cg) || dry)
+            ring_sweeps<RING_PREC, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, c0, x, TVec<T>::r(L), done, rz);
+        if (cg || dry)
+            ring_sweeps<RING_CGU, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, (const T*)nullptr, x,
+                                              TVec<T>::r(L), done, rz, cg);
+        if ((!c0 && !cg) || dry)
             ring_sweeps<RING_PRE, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, (const T*)nullptr, x,
-                                              TVec<T>::r(L), done);
+                                              TVec<T>::r(L), done, rz);
     } else if (s >= 2 && c0 && !cg) {   // the first iterate formed by the caller
         vct<VC_PREC, V, T, B, T>(ctx, dry, tA, err, dinv, omega, b, c0, x, done);
     } else if (s >= 2) {
@@ -1819,8 +1864,12 @@ static bool cg_update_fused() {
     const char* e = std::getenv("CFA_CG_FUSE_UPDATE");
     return e && e[0] == '1';
 }
+bool amg_on_rings(const cfa_amg* amg) {
+    return amg && amg->tiled && !amg->levels.empty() && amg->levels[0].ring.ok;
+}
 bool amg_can_fuse_update(const cfa_amg* amg) {
-    return cg_update_fused() && amg && !(!amg->levels.empty() && amg->levels[0].ring.ok) && !amg->levels.empty() && amg->tiled && amg->opts.smooth_steps == 2 &&
+    if (amg_on_rings(amg)) return true;
+    return cg_update_fused() && amg && !amg->levels.empty() && amg->tiled && amg->opts.smooth_steps == 2 &&
            !amg->levels[0].fusedQ;
 }
 

@@ -172,11 +172,17 @@ struct RzFuse {
     const double* alpha;
     double* part;
     unsigned int* counter;
+    // the CG's residual when its update rides in the V-cycle on ring tiles (CgFuse::r_alt): r_alt
+    // after an odd number of iterations, else the V-cycle's r. Both null: always r
+    const double* r_alt;
+    const int* iter;
 };
 // The CG's update before the preconditioner (x += alpha pn, r -= alpha q, p = pn, |r| and the
 // stopping test) folded into the V-cycle's level-0 kernels: the pre-smoothing sweep gathers
 // r - alpha q for its right-hand side, the residual pass (which reads only its own rows) writes
-// the new r, x and p and finishes |r| as the CG's update kernel would.
+// the new r, x and p and finishes |r| as the CG's update kernel would. On ring tiles one kernel does
+// all of it; other blocks still gather the old residual then, so the new one goes to the other of
+// two buffers, r and r_alt, by the iteration's parity.
 struct CgFuse {
     double* r;
     const double* q;
@@ -187,10 +193,13 @@ struct CgFuse {
     double* part;
     unsigned int* counter;
     CondArg cond;
+    double* r_alt;
 };
-// Whether amg_vcycle_rz takes the CG's update (CFA_CG_FUSE_UPDATE=1, a tile-streamed hierarchy
-// with two smoothing steps and level 0's residual pass unfused).
+// Whether amg_vcycle_rz takes the CG's update: level 0 on ring tiles, or CFA_CG_FUSE_UPDATE=1 and a
+// tile-streamed hierarchy with two smoothing steps and level 0's residual pass unfused.
 bool amg_can_fuse_update(const cfa_amg* amg);
+// Level 0 runs on ring tiles (small systems, ring.cu).
+bool amg_on_rings(const cfa_amg* amg);
 // The level-0 pre-smoothing's scaling: its first iterate is c = omega0 D0^-1 r in the V-cycle's
 // level-0 vector type (fp32: float), which a caller that writes r anyway can form (dinv, omega)
 // so that the pre-smoothing gathers c alone. False where the V-cycle does not take c (not

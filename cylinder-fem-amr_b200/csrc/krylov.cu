@@ -1199,7 +1199,7 @@ struct SegGraph {
 
 struct PcgWork {
     int cap = 0;
-    DevBuf<double> x, r, z, p, pn, q, gx, gy, dinv;
+    DevBuf<double> x, r, r2, z, p, pn, q, gx, gy, dinv;   // r2: RzFuse::r_alt
     DevBuf<double> c0;                 // omega0 D0^-1 r for the V-cycle's level 0 (float or double elements)
     DevBuf<CgState> st;
     // tile-streamed copy of the operator: K - B^T M^-1 B as one matrix on the two-ring pattern
@@ -1318,6 +1318,12 @@ static cfa_status build_graph(cfa_ctx* ctx, GraphCache& gc, Init init, Body body
     CFA_CUDA(cudaGraphInstantiate(&gc.exec, g, 0));
     return CFA_OK;
 }
+
+// Iterations per pass of a PCG loop's WHILE node. A pass costs 2 to 3 us beside its kernels, which
+// two iterations share; an iteration past the stop returns at each kernel's first read. Small systems
+// gain (8k vertices 2.68 -> 2.55 ms per 69 iterations); at 402k vertices the skipped kernels' early
+// tile copies cost more (8.69 -> 8.93 ms).
+static int pcg_iters_per_pass(const cfa_amg* amg) { return amg_on_rings(amg) ? 2 : 1; }
 
 template <class S>
 static cfa_status loop_enter(cfa_ctx* ctx, const S* st, CondArg cond) {
@@ -1529,6 +1535,13 @@ static bool split_p(const cfa_ctx* ctx, const PcgWork& W, const PcgArgs& a) {
            (long long)a.n > 512LL * ctx->num_sms;
 }
 
+static RzFuse rz_fuse(PcgWork& W, const PcgArgs& a, int flexible) {
+    CgState* st = W.st.p;
+    const bool two = amg_on_rings(a.amg);   // its update alternates between two residual buffers
+    return {W.q.p, flexible, &st->rz, &st->beta, &st->alpha, W.part.p, W.counter.p, two ? W.r2.p : nullptr,
+            two ? &st->iter : nullptr};
+}
+
 static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piece, CondArg cond) {
     const int n = a.n;
     const int gv = row_grid(ctx, n, 1);
@@ -1574,8 +1587,8 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
             if (!a.prec) {
                 // z = M^-1 r with r.z (and z.q) folded into the V-cycle's last sweep where it can be
                 const int flexible = pcg_flexible(a.amg);
-                const RzFuse f{W.q.p, flexible, &st->rz, &st->beta, &st->alpha, W.part.p, W.counter.p};
-                const CgFuse g{W.r.p, W.q.p, W.pn.p, W.x.p, W.p.p, st, W.part.p, W.counter.p, cond};
+                const RzFuse f = rz_fuse(W, a, flexible);
+                const CgFuse g{W.r.p, W.q.p, W.pn.p, W.x.p, W.p.p, st, W.part.p, W.counter.p, cond, W.r2.p};
                 bool fused = false;
                 CFA_PROPAGATE(amg_vcycle_rz(ctx, a.amg, W.r.p, W.z.p, done, f, &fused, fuse_update ? &g : nullptr,
                                             prescale ? (const void*)W.c0.p : nullptr, a.vc64 != 0));
@@ -1622,7 +1635,7 @@ static cfa_status pcg_resume(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, double 
     const int* done = &st->done;
     CFA_LAUNCH(ctx, k_cg_phase, 1, 32, 0, st, tol, cond);
     const int flexible = pcg_flexible(a.amg);
-    const RzFuse f{W.q.p, flexible, &st->rz, &st->beta, &st->alpha, W.part.p, W.counter.p};
+    const RzFuse f = rz_fuse(W, a, flexible);
     bool fused = false;
     CFA_PROPAGATE(amg_vcycle_rz(ctx, a.amg, W.r.p, W.z.p, done, f, &fused, nullptr, nullptr, a.vc64 != 0));
     if (!fused)
@@ -1643,6 +1656,11 @@ static cfa_status pcg_body(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, CondArg c
         CFA_PROPAGATE(pcg_piece(ctx, W, a, piece, cond));
         pcg_hook(a, W, piece);
     }
+    return CFA_OK;
+}
+
+static cfa_status pcg_pass(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, CondArg cond) {
+    for (int k = 0; k < pcg_iters_per_pass(a.amg); ++k) CFA_PROPAGATE(pcg_body(ctx, W, a, cond));
     return CFA_OK;
 }
 
@@ -1695,7 +1713,7 @@ static cfa_status ensure_pcg_vectors(cfa_ctx* ctx, PcgWork& W, int n) {
         W.graph.reset();
         W.graph2.reset();
         for (SegGraph& g : W.seg) g.reset();
-        for (DevBuf<double>* b : {&W.x, &W.r, &W.z, &W.p, &W.pn, &W.q, &W.gx, &W.gy, &W.dinv, &W.c0}) CFA_CUDA(b->ensure(n));
+        for (DevBuf<double>* b : {&W.x, &W.r, &W.r2, &W.z, &W.p, &W.pn, &W.q, &W.gx, &W.gy, &W.dinv, &W.c0}) CFA_CUDA(b->ensure(n));
         CFA_CUDA(W.st.ensure(1));
         CFA_CUDA(W.counter.ensure(1));
         CFA_CUDA(cudaMemsetAsync(W.counter.p, 0, sizeof(unsigned int), ctx->stream));
@@ -1881,7 +1899,7 @@ static cfa_status pcg_solve(cfa_ctx* ctx, const PcgArgs& a, cfa_solve_report* re
         GraphCache& g1 = W.graph.slot(key);
         if (!g1.exec || g1.key != key) {
             CFA_PROPAGATE(build_graph(ctx, g1, [&](CondArg c) { return loop_enter(ctx, W.st.p, c); },
-                                      [&](CondArg c) { return pcg_body(ctx, W, a1, c); }));
+                                      [&](CondArg c) { return pcg_pass(ctx, W, a1, c); }));
             g1.key = key;
         }
         CFA_CUDA(cudaGraphLaunch(g1.exec, ctx->stream));
@@ -1896,7 +1914,7 @@ static cfa_status pcg_solve(cfa_ctx* ctx, const PcgArgs& a, cfa_solve_report* re
             GraphCache& g2 = W.graph2.slot(key2);
             if (!g2.exec || g2.key != key2) {
                 CFA_PROPAGATE(build_graph(ctx, g2, [&](CondArg c) { return pcg_resume(ctx, W, a, a.tol, c); },
-                                          [&](CondArg c) { return pcg_body(ctx, W, a, c); }));
+                                          [&](CondArg c) { return pcg_pass(ctx, W, a, c); }));
                 g2.key = key2;
             }
             CFA_CUDA(cudaGraphLaunch(g2.exec, ctx->stream));
@@ -1938,7 +1956,8 @@ static cfa_status pcg_solve(cfa_ctx* ctx, const PcgArgs& a, cfa_solve_report* re
     }
     float ms = 0.f;
     CFA_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-    ctx->launches += extra_body * (long long)(h.iter + (h.status == CFA_BREAKDOWN ? 1 : 0));
+    const int per = pcg_iters_per_pass(a.amg);
+    ctx->launches += extra_body * (long long)((h.iter + (h.status == CFA_BREAKDOWN ? 1 : 0) + per - 1) / per);
     if (rep) {
         rep->iterations[0] = h.iter;
         rep->iterations[1] = 0;
