@@ -556,6 +556,7 @@ __global__ void k_inv_diag(int n, const int* __restrict__ rp, const int* __restr
 }
 
 // x += alpha pn, r -= alpha q, p = pn, ||r|| test (:237-247); JAC: z = D^-1 r and r.z -> beta
+// p null: pn is the direction itself, updated in place (k_cg_p).
 // SC (float or double, with JAC false): also c = omega0 D0^-1 r in the AMG's level-0 vector type,
 // the pre-smoothing's first iterate, which the V-cycle's level-0 pre-smoothing then gathers in
 // place of D0^-1 and r (PreScale); the product is formed as that pass forms it.
