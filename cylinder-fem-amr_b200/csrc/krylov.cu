@@ -2038,9 +2038,6 @@ static cfa_status plan_b2_tiles(cfa_ctx* ctx, B2Work& W, const B2Args& a) {
     std::vector<int> h_rp(a.n + 1);
     CFA_CUDA(cudaMemcpyAsync(h_rp.data(), a.rp, (a.n + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CFA_CUDA(cudaStreamSynchronize(ctx->stream));
-    // two stages: the third's shared memory holds more resident blocks instead, whose gathers hide the
-    // copies (402k vertices: momentum solve 2.40 -> 2.34 ms, 4.2M: 33.8 -> 32.2 ms)
-    W.tA.stages = 2;
     CFA_PROPAGATE(plan_tiled(ctx, h_rp.data(), a.n, 1, 8, W.tA));
     W.tile_key = key;
     W.tile_fp = fp;
