@@ -182,6 +182,7 @@ k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __rest
     __shared__ int uniq[kEtMaxInc];
     __shared__ int last_key[kEtThreads];
     __shared__ unsigned short rc[kEtMaxInc];
+    CFA_GRID_DEP();   // pos is the kernel before's output
     const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
     const int i0 = inc_ptr[r0], m = inc_ptr[r1] - i0;
     if (m > kEtMaxInc) {
