@@ -23,7 +23,7 @@ struct Geom {
 __device__ __forceinline__ Geom elem_geom(const int* nd, const double* __restrict__ x, const double* __restrict__ y) {
     Geom g;
     const double x0 = x[nd[0]], y0 = y[nd[0]], x1 = x[nd[1]], y1 = y[nd[1]], x2 = x[nd[2]], y2 = y[nd[2]];
-    const double detJ = (x1 - x0) * (y2 - y0) - (x2 - x0) * (y1 - y0);
+    const double detJ = __fma_rn(x1 - x0, y2 - y0, -__dmul_rn(x2 - x0, y1 - y0));
     g.area = 0.5 * fabs(detJ);
     g.ok = !(g.area < 1.0e-14);
     const double inv2A = 1.0 / (2.0 * g.area);
@@ -48,6 +48,76 @@ __device__ __forceinline__ double momentum_bc_u(int tag, double yi, double u_max
     if (tag == BC_INLET || tag == BC_OUTLET)
         return 4.0 * u_max * yi * (H - yi) / (H * H) * (tag == BC_OUTLET ? bc.outlet_scale : 1.0);
     return 0.0;
+}
+
+// Element terms of the momentum system (fem_kernels.cuh:88-176). Every product that meets a sum is
+// rounded explicitly: the two kernels below hold the same expressions in different surroundings, where
+// the compiler would contract them differently, and a last digit of A moves a mixed-precision solve
+// of some 500k vertices by up to 1e-8 (the ILU sweeps round their input to FP32).
+struct MomElem {
+    double area, area3, nu, tau, area_tau, area3_tau, skew_div, dpdx, dpdy;
+    double u_h[3], v_h[3], ugN[3];
+};
+__device__ __forceinline__ MomElem momentum_element(const int* nd, const Geom& g, const double* __restrict__ u_old,
+                                                    const double* __restrict__ v_old,
+                                                    const double* __restrict__ u_prev,
+                                                    const double* __restrict__ v_prev,
+                                                    const double* __restrict__ p_old,
+                                                    const double* __restrict__ nu_node, const MomParams& P,
+                                                    double inv_rho, double term_t) {
+    // reciprocals of the constant and per-launch divisors, taken once (the products differ from
+    // the quotients in the last bit at most; the element formula is division-bound in FP64)
+    constexpr double kThird = 1.0 / 3.0;
+    MomElem m;
+    m.area = g.area;
+    m.area3 = __dmul_rn(g.area, kThird);
+    double w_u = 0.0, w_v = 0.0, div_w = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double un = u_old[nd[k]], vn = v_old[nd[k]], um = u_prev[nd[k]], vm = v_prev[nd[k]];
+        m.u_h[k] = __fma_rn(P.a1, un, __dmul_rn(P.a2, um));
+        m.v_h[k] = __fma_rn(P.a1, vn, __dmul_rn(P.a2, vm));
+        const double wu = __fma_rn(P.c1, un, __dmul_rn(P.c2, um)), wv = __fma_rn(P.c1, vn, __dmul_rn(P.c2, vm));
+        w_u = __fma_rn(wu, kThird, w_u);
+        w_v = __fma_rn(wv, kThird, w_v);
+        div_w = __dadd_rn(div_w, __fma_rn(wu, g.dNdx[k], __dmul_rn(wv, g.dNdy[k])));
+    }
+    const double vel_mag = sqrt(__fma_rn(w_u, w_u, __dmul_rn(w_v, w_v))) + 1.0e-12;
+    const double h_K = sqrt(2.0 * g.area);
+    // element viscosity: the scalar nu, or the mean of a nodal field
+    m.nu = nu_node ? __dmul_rn(nu_node[nd[0]] + nu_node[nd[1]] + nu_node[nd[2]], kThird) : P.nu;
+    const double term_c = 2.0 * vel_mag / h_K;
+    const double term_d = 4.0 * m.nu / __dmul_rn(h_K, h_K);
+    m.tau = 1.0 / sqrt(__fma_rn(__dmul_rn(9.0, term_d), term_d, __fma_rn(term_c, term_c, __dmul_rn(term_t, term_t))));
+    m.area_tau = __dmul_rn(g.area, m.tau);
+    m.area3_tau = __dmul_rn(m.area3, m.tau);
+    m.skew_div = __dmul_rn(P.skew_coef, div_w);
+    const double p0 = p_old[nd[0]], p1 = p_old[nd[1]], p2 = p_old[nd[2]];
+    m.dpdx = __dmul_rn(__fma_rn(p2, g.dNdx[2], __fma_rn(p0, g.dNdx[0], __dmul_rn(p1, g.dNdx[1]))), inv_rho);
+    m.dpdy = __dmul_rn(__fma_rn(p2, g.dNdy[2], __fma_rn(p0, g.dNdy[0], __dmul_rn(p1, g.dNdy[1]))), inv_rho);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m.ugN[k] = __fma_rn(w_u, g.dNdx[k], __dmul_rn(w_v, g.dNdy[k]));
+    return m;
+}
+// A_aj of one element; f_u, f_v take its (M + Ms) u_h
+__device__ __forceinline__ double momentum_entry(const MomElem& m, double dNdx_a, double dNdy_a, double ugN_a,
+                                                 bool diag, int j, const Geom& g, double a0, double& f_u,
+                                                 double& f_v) {
+    constexpr double kSixth = 1.0 / 6.0, kTwelfth = 1.0 / 12.0;
+    const double M_ij = __dmul_rn(m.area, diag ? kSixth : kTwelfth);
+    const double MM = __dadd_rn(M_ij, __dmul_rn(m.area3_tau, ugN_a));
+    const double K_ij = __dmul_rn(m.area, __fma_rn(dNdx_a, g.dNdx[j], __dmul_rn(dNdy_a, g.dNdy[j])));
+    const double C_ij = __fma_rn(m.skew_div, M_ij, __dmul_rn(m.area3, m.ugN[j]));
+    f_u = __fma_rn(MM, m.u_h[j], f_u);
+    f_v = __fma_rn(MM, m.v_h[j], f_v);
+    return __fma_rn(__dmul_rn(m.area_tau, ugN_a), m.ugN[j],
+                    __dadd_rn(__fma_rn(m.nu, K_ij, __dmul_rn(a0, MM)), C_ij));
+}
+// the pressure gradient's share of f_u, f_v
+__device__ __forceinline__ void momentum_pressure(const MomElem& m, double ugN_a, double& f_u, double& f_v) {
+    const double tw = __dadd_rn(m.area3, __dmul_rn(m.area_tau, ugN_a));
+    f_u = __fma_rn(-tw, m.dpdx, f_u);
+    f_v = __fma_rn(-tw, m.dpdy, f_v);
 }
 
 // Momentum rows: k_assemble_momentum_fem (fem_kernels.cuh:40-181) gathered per row, lumped mass,
@@ -83,62 +153,24 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
         }
     }
     double f_u_row = 0.0, f_v_row = 0.0, m_row = 0.0;
-    // reciprocals of the constant and per-launch divisors, taken once (the products differ from
-    // the quotients in the last bit at most; the element formula is division-bound in FP64)
-    constexpr double kThird = 1.0 / 3.0, kSixth = 1.0 / 6.0, kTwelfth = 1.0 / 12.0;
-    const double inv_rho = 1.0 / P.rho, term_t_p = 2.0 / P.tau_time;
+    const double inv_rho = 1.0 / P.rho, term_t = 2.0 / P.tau_time;
     for (int s = inc_ptr[i]; s < inc_ptr[i + 1]; ++s) {
         const int e = inc[s] >> 2, a = inc[s] & 3;
         int nd[3];
         load_elem(ev, e, nd);
         const Geom g = elem_geom(nd, x, y);
         if (!g.ok) continue;
-        const double area = g.area;
-        const double area3 = area * kThird;
-        m_row += area3;
+        m_row = __dadd_rn(m_row, __dmul_rn(g.area, 1.0 / 3.0));
         if (dir) continue;
-        double u_h[3], v_h[3], w_u = 0.0, w_v = 0.0, div_w = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double un = u_old[nd[k]], vn = v_old[nd[k]], um = u_prev[nd[k]], vm = v_prev[nd[k]];
-            u_h[k] = P.a1 * un + P.a2 * um;
-            v_h[k] = P.a1 * vn + P.a2 * vm;
-            const double wu = P.c1 * un + P.c2 * um, wv = P.c1 * vn + P.c2 * vm;
-            w_u += wu * kThird;
-            w_v += wv * kThird;
-            div_w += wu * g.dNdx[k] + wv * g.dNdy[k];
-        }
-        const double vel_mag = sqrt(w_u * w_u + w_v * w_v) + 1.0e-12;
-        const double h_K = sqrt(2.0 * area);
-        // element viscosity: the scalar nu, or the mean of a nodal field
-        const double nu = nu_node ? (nu_node[nd[0]] + nu_node[nd[1]] + nu_node[nd[2]]) * kThird : P.nu;
-        const double term_t = term_t_p;
-        const double term_c = 2.0 * vel_mag / h_K;
-        const double term_d = 4.0 * nu / (h_K * h_K);
-        const double tau_supg = 1.0 / sqrt(term_t * term_t + term_c * term_c + 9.0 * term_d * term_d);
-        const double p0 = p_old[nd[0]], p1 = p_old[nd[1]], p2 = p_old[nd[2]];
-        const double dpdx = (p0 * g.dNdx[0] + p1 * g.dNdx[1] + p2 * g.dNdx[2]) * inv_rho;
-        const double dpdy = (p0 * g.dNdy[0] + p1 * g.dNdy[1] + p2 * g.dNdy[2]) * inv_rho;
-        double ugN[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ugN[k] = w_u * g.dNdx[k] + w_v * g.dNdy[k];
+        const MomElem m = momentum_element(nd, g, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, inv_rho, term_t);
         double f_u = 0.0, f_v = 0.0;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const double M_ij = (a == j) ? (area * kSixth) : (area * kTwelfth);
-            const double K_ij = area * (g.dNdx[a] * g.dNdx[j] + g.dNdy[a] * g.dNdy[j]);
-            const double C_ij = area3 * ugN[j] + P.skew_coef * div_w * M_ij;
-            const double S_ij = area * tau_supg * ugN[a] * ugN[j];
-            const double Ms_ij = area3 * tau_supg * ugN[a];
-            const double A_ij = P.a0 * (M_ij + Ms_ij) + nu * K_ij + C_ij + S_ij;
+            const double A_ij = momentum_entry(m, g.dNdx[a], g.dNdy[a], m.ugN[a], a == j, j, g, P.a0, f_u, f_v);
             const int p = pos[3 * s + j];
             if (local) acc[(p - r0) * T] += A_ij; else A_val[p] += A_ij;
-            f_u += (M_ij + Ms_ij) * u_h[j];
-            f_v += (M_ij + Ms_ij) * v_h[j];
         }
-        const double tw = area3 + area * tau_supg * ugN[a];
-        f_u -= tw * dpdx;
-        f_v -= tw * dpdy;
+        momentum_pressure(m, m.ugN[a], f_u, f_v);
         f_u_row += f_u;
         f_v_row += f_v;
     }
@@ -174,7 +206,6 @@ k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const doubl
     const EtBlock b = et_block(tv, n);
     const int S = tv.stride;
     CFA_GRID_DEP();
-    constexpr double kThird = 1.0 / 3.0, kSixth = 1.0 / 6.0, kTwelfth = 1.0 / 12.0;
     const double inv_rho = 1.0 / P.rho, term_t = 2.0 / P.tau_time;
     for (int le = threadIdx.x; le < b.ne; le += kEtThreads) {
         int nd[3];
@@ -186,50 +217,19 @@ k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const doubl
             for (int q = 0; q < 16; ++q) rec[q * S] = 0.0;
             continue;
         }
-        const double area = g.area, area3 = area * kThird;
-        double u_h[3], v_h[3], w_u = 0.0, w_v = 0.0, div_w = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double un = u_old[nd[k]], vn = v_old[nd[k]], um = u_prev[nd[k]], vm = v_prev[nd[k]];
-            u_h[k] = P.a1 * un + P.a2 * um;
-            v_h[k] = P.a1 * vn + P.a2 * vm;
-            const double wu = P.c1 * un + P.c2 * um, wv = P.c1 * vn + P.c2 * vm;
-            w_u += wu * kThird;
-            w_v += wv * kThird;
-            div_w += wu * g.dNdx[k] + wv * g.dNdy[k];
-        }
-        const double vel_mag = sqrt(w_u * w_u + w_v * w_v) + 1.0e-12;
-        const double h_K = sqrt(2.0 * area);
-        // element viscosity: the scalar nu, or the mean of a nodal field
-        const double nu = nu_node ? (nu_node[nd[0]] + nu_node[nd[1]] + nu_node[nd[2]]) * kThird : P.nu;
-        const double term_c = 2.0 * vel_mag / h_K;
-        const double term_d = 4.0 * nu / (h_K * h_K);
-        const double tau_supg = 1.0 / sqrt(term_t * term_t + term_c * term_c + 9.0 * term_d * term_d);
-        const double p0 = p_old[nd[0]], p1 = p_old[nd[1]], p2 = p_old[nd[2]];
-        const double dpdx = (p0 * g.dNdx[0] + p1 * g.dNdx[1] + p2 * g.dNdx[2]) * inv_rho;
-        const double dpdy = (p0 * g.dNdy[0] + p1 * g.dNdy[1] + p2 * g.dNdy[2]) * inv_rho;
-        double ugN[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ugN[k] = w_u * g.dNdx[k] + w_v * g.dNdy[k];
+        const MomElem m = momentum_element(nd, g, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, inv_rho, term_t);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             double f_u = 0.0, f_v = 0.0;
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const double M_ij = (a == j) ? (area * kSixth) : (area * kTwelfth);
-                const double K_ij = area * (g.dNdx[a] * g.dNdx[j] + g.dNdy[a] * g.dNdy[j]);
-                const double C_ij = area3 * ugN[j] + P.skew_coef * div_w * M_ij;
-                const double S_ij = area * tau_supg * ugN[a] * ugN[j];
-                const double Ms_ij = area3 * tau_supg * ugN[a];
-                rec[(3 * a + j) * S] = P.a0 * (M_ij + Ms_ij) + nu * K_ij + C_ij + S_ij;
-                f_u += (M_ij + Ms_ij) * u_h[j];
-                f_v += (M_ij + Ms_ij) * v_h[j];
-            }
-            const double tw = area3 + area * tau_supg * ugN[a];
-            rec[(9 + a) * S] = f_u - tw * dpdx;
-            rec[(12 + a) * S] = f_v - tw * dpdy;
+            for (int j = 0; j < 3; ++j)
+                rec[(3 * a + j) * S] =
+                    momentum_entry(m, g.dNdx[a], g.dNdy[a], m.ugN[a], a == j, j, g, P.a0, f_u, f_v);
+            momentum_pressure(m, m.ugN[a], f_u, f_v);
+            rec[(9 + a) * S] = f_u;
+            rec[(12 + a) * S] = f_v;
         }
-        rec[15 * S] = area3;
+        rec[15 * S] = m.area3;
     }
     __syncthreads();
     const int p0 = rp[b.r0], p1 = rp[b.r1];

@@ -157,3 +157,76 @@ def test_node_gradients_match_the_formulas(name):
     ud = u - 6.0 * m.y * (1 - m.y)
     for k, e in enumerate((*grad(ud), *grad(v))):
         close(rec[k * n:(k + 1) * n], nodes(w * e))
+
+
+# ----------------------------------------------------------------------------------------------
+# the two forms give the same bits
+# ----------------------------------------------------------------------------------------------
+HUB = 2000   # elements around one vertex, whose records exceed a tile: the whole mesh takes the row gathers
+
+
+def _with_hub(m):
+    """`m` and, apart from it, a disc of HUB elements: m's rows as the gathers form them."""
+    w = _wheel(HUB)
+    return F.Mesh(np.concatenate([m.x, w.x]), np.concatenate([m.y, w.y]), np.concatenate([m.tag, 0 * w.tag]).astype(np.int32),
+                  np.concatenate([m.tri, w.tri + m.n]).astype(np.int32), np.concatenate([m.gen, w.gen]))
+
+
+class _Pair:
+    """A mesh on the device alone (element tiles) and with the hub (row gathers), the same fields on both."""
+
+    def __init__(self, m):
+        import torch
+        import cfa_b200 as cfa
+        from oracle import oracle as O
+        self.m, self.ctx, self.dms = m, cfa.default_context(), []
+        for mesh in (m, _with_hub(m)):
+            rp, ci = O.csr_build(mesh.n, mesh.elem_v)
+            self.dms.append(cfa.DeviceMesh(self.ctx, mesh, torch.from_numpy(rp).to("cuda"), torch.from_numpy(ci).to("cuda")))
+        self.n, self.nnz, self.ne = m.n, self.dms[0].nnz, m.ne
+
+    def fields(self, k, *values):
+        """The values (per vertex, or per element) as device arrays of mesh k, filled up for the hub."""
+        import torch
+        dm, out = self.dms[k], []
+        for a in values:
+            size = dm.ne if len(a) == self.ne else dm.n
+            out.append(torch.from_numpy(np.concatenate([a, np.full(size - len(a), 0.7)])).to("cuda"))
+        return out
+
+    def same(self, call):
+        """call(dm, k) -> output tensors, for both forms; their parts that belong to m are compared."""
+        import torch
+        outs = [call(dm, k) for k, dm in enumerate(self.dms)]
+        for q, (a, b) in enumerate(zip(*outs)):
+            blocks = 4 if a.numel() in (4 * self.n, 4 * self.nnz) else 1
+            a, b = a.view(blocks, -1), b.view(blocks, -1)
+            assert torch.isfinite(a).all()
+            assert torch.equal(a, b[:, :a.shape[1]]), q
+
+
+BIT_MESHES = {"one": _one, "tiny": lambda: F.make_mesh("tiny"), "small": lambda: F.make_mesh("small"),
+              "small_shuffled": lambda: _shuffled(F.make_mesh("small")), "c0": lambda: F.make_mesh("c0"),
+              "medium": lambda: F.make_mesh("medium")}
+
+
+def _empty(k):
+    import torch
+    return torch.full((k,), float("nan"), dtype=torch.float64, device="cuda")
+
+
+@pytest.mark.parametrize("with_nu", [False, True])
+@pytest.mark.parametrize("name", list(BIT_MESHES))
+def test_momentum_tiles_give_the_gathers_bits(name, with_nu):
+    import cfa_b200 as cfa
+    p = _Pair(BIT_MESHES[name]())
+    f = [F.fourier_field(p.m.x, p.m.y, k) for k in range(1, 5)]
+    for prm in (cfa.bdf2_params(), cfa.bdf2_params(bdf2=False, skew=0.3, rho=1.3)):
+        for u_max in (None, 1.5):
+            def call(dm, k):
+                u, v, um, vm, pr, nu = p.fields(k, f[0], f[1], 0.9 * f[0], 1.1 * f[1], 0.3 * f[2], 1e-3 * (1 + 0.1 * f[3]))
+                out = [_empty(dm.nnz), _empty(dm.n), _empty(dm.n), _empty(dm.n)]
+                bc = {} if u_max is None else {"u": u.clone(), "v": v.clone(), "u_max": u_max}
+                cfa.assemble_momentum(p.ctx, dm, u, v, um, vm, pr, prm, *out, nu_node=nu if with_nu else None, **bc)
+                return out
+            p.same(call)
