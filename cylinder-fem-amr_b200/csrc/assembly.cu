@@ -56,7 +56,7 @@ __device__ __forceinline__ double momentum_bc_u(int tag, double yi, double u_max
 // of some 500k vertices by up to 1e-8 (the ILU sweeps round their input to FP32).
 struct MomElem {
     double area, area3, nu, tau, area_tau, area3_tau, skew_div, dpdx, dpdy;
-    double u_h[3], v_h[3], ugN[3];
+    double u_h[3], v_h[3];
 };
 __device__ __forceinline__ MomElem momentum_element(const int* nd, const Geom& g, const double* __restrict__ u_old,
                                                     const double* __restrict__ v_old,
@@ -64,7 +64,7 @@ __device__ __forceinline__ MomElem momentum_element(const int* nd, const Geom& g
                                                     const double* __restrict__ v_prev,
                                                     const double* __restrict__ p_old,
                                                     const double* __restrict__ nu_node, const MomParams& P,
-                                                    double inv_rho, double term_t) {
+                                                    double inv_rho, double term_t, double (&ugN)[3]) {
     // reciprocals of the constant and per-launch divisors, taken once (the products differ from
     // the quotients in the last bit at most; the element formula is division-bound in FP64)
     constexpr double kThird = 1.0 / 3.0;
@@ -96,21 +96,21 @@ __device__ __forceinline__ MomElem momentum_element(const int* nd, const Geom& g
     m.dpdx = __dmul_rn(__fma_rn(p2, g.dNdx[2], __fma_rn(p0, g.dNdx[0], __dmul_rn(p1, g.dNdx[1]))), inv_rho);
     m.dpdy = __dmul_rn(__fma_rn(p2, g.dNdy[2], __fma_rn(p0, g.dNdy[0], __dmul_rn(p1, g.dNdy[1]))), inv_rho);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) m.ugN[k] = __fma_rn(w_u, g.dNdx[k], __dmul_rn(w_v, g.dNdy[k]));
+    for (int k = 0; k < 3; ++k) ugN[k] = __fma_rn(w_u, g.dNdx[k], __dmul_rn(w_v, g.dNdy[k]));
     return m;
 }
 // A_aj of one element; f_u, f_v take its (M + Ms) u_h
 __device__ __forceinline__ double momentum_entry(const MomElem& m, double dNdx_a, double dNdy_a, double ugN_a,
-                                                 bool diag, int j, const Geom& g, double a0, double& f_u,
-                                                 double& f_v) {
+                                                 bool diag, int j, const Geom& g, double ugN_j, double a0,
+                                                 double& f_u, double& f_v) {
     constexpr double kSixth = 1.0 / 6.0, kTwelfth = 1.0 / 12.0;
     const double M_ij = __dmul_rn(m.area, diag ? kSixth : kTwelfth);
     const double MM = __dadd_rn(M_ij, __dmul_rn(m.area3_tau, ugN_a));
     const double K_ij = __dmul_rn(m.area, __fma_rn(dNdx_a, g.dNdx[j], __dmul_rn(dNdy_a, g.dNdy[j])));
-    const double C_ij = __fma_rn(m.skew_div, M_ij, __dmul_rn(m.area3, m.ugN[j]));
+    const double C_ij = __fma_rn(m.skew_div, M_ij, __dmul_rn(m.area3, ugN_j));
     f_u = __fma_rn(MM, m.u_h[j], f_u);
     f_v = __fma_rn(MM, m.v_h[j], f_v);
-    return __fma_rn(__dmul_rn(m.area_tau, ugN_a), m.ugN[j],
+    return __fma_rn(__dmul_rn(m.area_tau, ugN_a), ugN_j,
                     __dadd_rn(__fma_rn(m.nu, K_ij, __dmul_rn(a0, MM)), C_ij));
 }
 // the pressure gradient's share of f_u, f_v
@@ -162,15 +162,17 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
         if (!g.ok) continue;
         m_row = __dadd_rn(m_row, __dmul_rn(g.area, 1.0 / 3.0));
         if (dir) continue;
-        const MomElem m = momentum_element(nd, g, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, inv_rho, term_t);
+        double ugN[3];
+        const MomElem m =
+            momentum_element(nd, g, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, inv_rho, term_t, ugN);
         double f_u = 0.0, f_v = 0.0;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const double A_ij = momentum_entry(m, g.dNdx[a], g.dNdy[a], m.ugN[a], a == j, j, g, P.a0, f_u, f_v);
+            const double A_ij = momentum_entry(m, g.dNdx[a], g.dNdy[a], ugN[a], a == j, j, g, ugN[j], P.a0, f_u, f_v);
             const int p = pos[3 * s + j];
             if (local) acc[(p - r0) * T] += A_ij; else A_val[p] += A_ij;
         }
-        momentum_pressure(m, m.ugN[a], f_u, f_v);
+        momentum_pressure(m, ugN[a], f_u, f_v);
         f_u_row += f_u;
         f_v_row += f_v;
     }
@@ -194,7 +196,9 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
 // Dirichlet rows. Bound by latency: each block's chain of plan, vertices and fields, the divisions
 // and square roots of the element formula, then the entries' codes. Against the row gather: 142 ->
 // 130 us at 402k vertices (130 MB, 1.0 TB/s), 21.0 -> 13.3 us at 22.5k, 19.5 -> 13.2 us at 8k.
-__global__ void __launch_bounds__(kEtThreads)
+// Three blocks per SM (80 registers) matter: at 92 registers, two blocks, 189 against 144 us at 402k
+// vertices, each with the L2 flushed first.
+__global__ void __launch_bounds__(kEtThreads, 3)
 k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
                  const double* __restrict__ y, const int* __restrict__ tag, const int* __restrict__ rp,
                  const int* __restrict__ ci, const double* __restrict__ u_old, const double* __restrict__ v_old,
@@ -217,15 +221,17 @@ k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const doubl
             for (int q = 0; q < 16; ++q) rec[q * S] = 0.0;
             continue;
         }
-        const MomElem m = momentum_element(nd, g, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, inv_rho, term_t);
+        double ugN[3];
+        const MomElem m =
+            momentum_element(nd, g, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, inv_rho, term_t, ugN);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             double f_u = 0.0, f_v = 0.0;
 #pragma unroll
             for (int j = 0; j < 3; ++j)
                 rec[(3 * a + j) * S] =
-                    momentum_entry(m, g.dNdx[a], g.dNdy[a], m.ugN[a], a == j, j, g, P.a0, f_u, f_v);
-            momentum_pressure(m, m.ugN[a], f_u, f_v);
+                    momentum_entry(m, g.dNdx[a], g.dNdy[a], ugN[a], a == j, j, g, ugN[j], P.a0, f_u, f_v);
+            momentum_pressure(m, ugN[a], f_u, f_v);
             rec[(9 + a) * S] = f_u;
             rec[(12 + a) * S] = f_v;
         }
