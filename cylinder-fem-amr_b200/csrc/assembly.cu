@@ -355,6 +355,45 @@ __global__ void k_scalar_gradient_rows(int n, const int* __restrict__ ev, const 
     gy_out[i] = sy;
 }
 
+// Element terms of the pressure system (fem_kernels.cuh:230-270), rounded explicitly as the momentum's
+// are: the row gather and the element tiles give the same bits whatever the compiler contracts.
+__device__ __forceinline__ double pressure_divergence(const int* nd, const Geom& g, const double* __restrict__ us,
+                                                      const double* __restrict__ vs) {
+    double d = __fma_rn(us[nd[0]], g.dNdx[0], __dmul_rn(us[nd[1]], g.dNdx[1]));
+    d = __fma_rn(us[nd[2]], g.dNdx[2], d);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) d = __fma_rn(vs[nd[q]], g.dNdy[q], d);
+    return d;
+}
+// grad p and the projected gradient of one element
+__device__ __forceinline__ void pressure_gradients(const int* nd, const Geom& g, const double* __restrict__ p_old,
+                                                   const double* __restrict__ gpx, const double* __restrict__ gpy,
+                                                   const double* __restrict__ mass, double s, double& gx, double& gy,
+                                                   double& sx, double& sy) {
+    const double p0 = p_old[nd[0]], p1 = p_old[nd[1]], p2 = p_old[nd[2]], third = sqrt(s) / 3.0;
+    gx = __fma_rn(p2, g.dNdx[2], __fma_rn(p0, g.dNdx[0], __dmul_rn(p1, g.dNdx[1])));
+    gy = __fma_rn(p2, g.dNdy[2], __fma_rn(p0, g.dNdy[0], __dmul_rn(p1, g.dNdy[1])));
+    sx = sy = 0.0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double im = 1.0 / fmax(mass[nd[q]], 1.0e-14);
+        sx = __fma_rn(gpx[nd[q]], im, sx);
+        sy = __fma_rn(gpy[nd[q]], im, sy);
+    }
+    sx = __dmul_rn(sx, third);
+    sy = __dmul_rn(sy, third);
+}
+// -(rho / dt) (area / 3) div u - (s area (grad N . grad p) - area (grad N . the projected gradient))
+__device__ __forceinline__ double pressure_rhs(double area, double s, double rho_dt, double div_u, double dNdx_a,
+                                               double dNdy_a, double gx, double gy, double sx, double sy) {
+    const double stab_i = __fma_rn(__dmul_rn(s, area), __fma_rn(dNdx_a, gx, __dmul_rn(dNdy_a, gy)),
+                                   -__dmul_rn(area, __fma_rn(dNdy_a, sy, __dmul_rn(dNdx_a, sx))));
+    return __fma_rn(__dmul_rn(-rho_dt, area / 3.0), div_u, -stab_i);
+}
+__device__ __forceinline__ double pressure_entry(double area, double xa, double ya, double xb, double yb) {
+    return __dmul_rn(area, __fma_rn(xa, xb, __dmul_rn(ya, yb)));
+}
+
 // Pressure rows: k_assemble_pressure_poisson (fem_kernels.cuh:201-282) gathered per row; with
 // oss_val the rows of B and B^T of k_assemble_oss_operator (:807-847) and inv_m (:849-852) in
 // the same pass; with with_bc the Dirichlet rows/columns of k_apply_bc_pressure (:460-490).
@@ -408,50 +447,38 @@ k_pressure_rows(int n, int nnz, const int* __restrict__ ev, const double* __rest
         const Geom g = elem_geom(nd, x, y);
         if (!g.ok) continue;
         const double area = g.area;
-        const double div_u = us[nd[0]] * g.dNdx[0] + us[nd[1]] * g.dNdx[1] + us[nd[2]] * g.dNdx[2]
-                           + vs[nd[0]] * g.dNdy[0] + vs[nd[1]] * g.dNdy[1] + vs[nd[2]] * g.dNdy[2];
-        const double rhs_contrib = -(rho / dt) * (area / 3.0) * div_u;
+        const double div_u = pressure_divergence(nd, g, us, vs);
         double s = 0.0, sx = 0.0, sy = 0.0, gx = 0.0, gy = 0.0;
         if (stab > 0.0) {
             s = elem_s[e];
-            const double rs = sqrt(s);
-            gx = p_old[nd[0]] * g.dNdx[0] + p_old[nd[1]] * g.dNdx[1] + p_old[nd[2]] * g.dNdx[2];
-            gy = p_old[nd[0]] * g.dNdy[0] + p_old[nd[1]] * g.dNdy[1] + p_old[nd[2]] * g.dNdy[2];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const double im = 1.0 / fmax(mass[nd[q]], 1.0e-14);
-                sx += gpx[nd[q]] * im;
-                sy += gpy[nd[q]] * im;
-            }
-            sx *= rs / 3.0;
-            sy *= rs / 3.0;
+            pressure_gradients(nd, g, p_old, gpx, gpy, mass, s, gx, gy, sx, sy);
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const double K_ij = area * (g.dNdx[a] * g.dNdx[j] + g.dNdy[a] * g.dNdy[j]);
+            const double K_ij = pressure_entry(area, g.dNdx[a], g.dNdy[a], g.dNdx[j], g.dNdy[j]);
             const int p = pos[3 * k + j];
-            if (local) sK[(p - r0) * T] += (1.0 + s) * K_ij; else Kp_val[p] += (1.0 + s) * K_ij;
+            if (local) sK[(p - r0) * T] = __fma_rn(1.0 + s, K_ij, sK[(p - r0) * T]);
+            else Kp_val[p] = __fma_rn(1.0 + s, K_ij, Kp_val[p]);
         }
-        const double stab_i = s * area * (g.dNdx[a] * gx + g.dNdy[a] * gy) - area * (g.dNdx[a] * sx + g.dNdy[a] * sy);
-        rhs_row += rhs_contrib - stab_i;
-        div_row += (area / 3.0) * div_u;
+        rhs_row += pressure_rhs(area, s, rho / dt, div_u, g.dNdx[a], g.dNdy[a], gx, gy, sx, sy);
+        div_row = __fma_rn(area / 3.0, div_u, div_row);
         if (want_oss) {
-            const double w = sqrt(elem_s[e]) * area / 3.0;
+            const double w = __dmul_rn(sqrt(elem_s[e]), area) / 3.0;
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 const int p = pos[3 * k + j];
                 // B_ij = sum_K w_K grad N_j|K (row i, column j); B^T_ij = B_ji = sum_K w_K grad N_i|K
                 if (local) {
                     const int q = (p - r0) * T;
-                    sBx[q] += w * g.dNdx[j];
-                    sBy[q] += w * g.dNdy[j];
-                    sTx[q] += w * g.dNdx[a];
-                    sTy[q] += w * g.dNdy[a];
+                    sBx[q] = __fma_rn(w, g.dNdx[j], sBx[q]);
+                    sBy[q] = __fma_rn(w, g.dNdy[j], sBy[q]);
+                    sTx[q] = __fma_rn(w, g.dNdx[a], sTx[q]);
+                    sTy[q] = __fma_rn(w, g.dNdy[a], sTy[q]);
                 } else {
-                    Bx[p] += w * g.dNdx[j];
-                    By[p] += w * g.dNdy[j];
-                    BTx[p] += w * g.dNdx[a];
-                    BTy[p] += w * g.dNdy[a];
+                    Bx[p] = __fma_rn(w, g.dNdx[j], Bx[p]);
+                    By[p] = __fma_rn(w, g.dNdy[j], By[p]);
+                    BTx[p] = __fma_rn(w, g.dNdx[a], BTx[p]);
+                    BTy[p] = __fma_rn(w, g.dNdy[a], BTy[p]);
                 }
             }
         }
@@ -564,38 +591,22 @@ k_pressure_tiles(ElemTileView tv, int n, int nnz, const int* __restrict__ ev, co
             continue;
         }
         const double area = g.area;
-        const double div_u = us[nd[0]] * g.dNdx[0] + us[nd[1]] * g.dNdx[1] + us[nd[2]] * g.dNdx[2]
-                           + vs[nd[0]] * g.dNdy[0] + vs[nd[1]] * g.dNdy[1] + vs[nd[2]] * g.dNdy[2];
-        const double rs = sqrt(es);
+        const double div_u = pressure_divergence(nd, g, us, vs);
         double s = 0.0, sx = 0.0, sy = 0.0, gx = 0.0, gy = 0.0;
         if (stab > 0.0) {
             s = es;
-            gx = p_old[nd[0]] * g.dNdx[0] + p_old[nd[1]] * g.dNdx[1] + p_old[nd[2]] * g.dNdx[2];
-            gy = p_old[nd[0]] * g.dNdy[0] + p_old[nd[1]] * g.dNdy[1] + p_old[nd[2]] * g.dNdy[2];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const double im = 1.0 / fmax(mass[nd[q]], 1.0e-14);
-                sx = __fma_rn(gpx[nd[q]], im, sx);
-                sy = __fma_rn(gpy[nd[q]], im, sy);
-            }
-            sx *= rs / 3.0;
-            sy *= rs / 3.0;
+            pressure_gradients(nd, g, p_old, gpx, gpy, mass, s, gx, gy, sx, sy);
         }
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
 #pragma unroll
             for (int j = a; j < 3; ++j)   // 00 01 02 11 12 22
-                rec[(a + j + (a > 0 ? 1 : 0)) * S] = area * (g.dNdx[a] * g.dNdx[j] + g.dNdy[a] * g.dNdy[j]);
+                rec[(a + j + (a > 0 ? 1 : 0)) * S] = pressure_entry(area, g.dNdx[a], g.dNdy[a], g.dNdx[j], g.dNdy[j]);
             rec[(6 + a) * S] = g.dNdx[a];
             rec[(9 + a) * S] = g.dNdy[a];
-            // rhs - (s area (grad N . grad p) - area (grad N . the projection)), rounded explicitly:
-            // the PPE alone and the fused system give the same bits whatever the compiler contracts
-            const double stab_i =
-                __fma_rn(s * area, __fma_rn(g.dNdx[a], gx, __dmul_rn(g.dNdy[a], gy)),
-                         -__dmul_rn(area, __fma_rn(g.dNdx[a], sx, __dmul_rn(g.dNdy[a], sy))));
-            rec[(14 + a) * S] = __fma_rn(-(rho / dt) * (area / 3.0), div_u, -stab_i);
+            rec[(14 + a) * S] = pressure_rhs(area, s, rho / dt, div_u, g.dNdx[a], g.dNdy[a], gx, gy, sx, sy);
         }
-        rec[12 * S] = rs * area / 3.0;
+        rec[12 * S] = __dmul_rn(sqrt(es), area) / 3.0;
         rec[13 * S] = 1.0 + s;
         rec[17 * S] = area / 3.0;
         rec[18 * S] = div_u;

@@ -230,3 +230,38 @@ def test_momentum_tiles_give_the_gathers_bits(name, with_nu):
                 cfa.assemble_momentum(p.ctx, dm, u, v, um, vm, pr, prm, *out, nu_node=nu if with_nu else None, **bc)
                 return out
             p.same(call)
+
+
+@pytest.mark.parametrize("stab", [0.3, 0.0])
+@pytest.mark.parametrize("name", list(BIT_MESHES))
+def test_pressure_tiles_give_the_gathers_bits(name, stab):
+    import cfa_b200 as cfa
+    from oracle import oracle as O
+    p = _Pair(BIT_MESHES[name]())
+    m, dt = p.m, 2e-3 / 3
+    f = [F.fourier_field(m.x, m.y, k) for k in range(1, 4)]
+    s = O.oss_weights(m, f[0], f[1], dt, 1.0, 1e-3, 0.3)
+    mass = np.zeros(m.n)
+    np.add.at(mass, m.tri.ravel(), 1e-3 * (1.0 + np.arange(3 * m.ne) % 7))
+    g = [0.1 * mass * F.fourier_field(m.x, m.y, k) for k in (5, 6)]
+
+    def ppe(dm, k):
+        u, v, pr, gx, gy, ms, es = p.fields(k, *f, *g, mass, s)
+        out = [_empty(dm.nnz), _empty(dm.n), _empty(dm.n)]
+        cfa.assemble_ppe(p.ctx, dm, u, v, pr, gx, gy, ms, es, dt, 1.3, stab, *out, apply_bc=False)
+        return out
+
+    def oss(dm, k):
+        ms, es = p.fields(k, mass, s)
+        out = [_empty(4 * dm.nnz), _empty(dm.n)]
+        cfa.assemble_oss(p.ctx, dm, es, ms, *out)
+        return out
+
+    def system(dm, k):   # Dirichlet rows and columns in the same pass
+        u, v, pr, gx, gy, ms, es, dp = p.fields(k, *f, *g, mass, s, f[2])
+        out = [_empty(dm.nnz), _empty(dm.n), _empty(dm.n), dp, _empty(4 * dm.nnz), _empty(dm.n)]
+        cfa.assemble_pressure_system(p.ctx, dm, u, v, pr, gx, gy, ms, es, dt, 1.3, stab, *out)
+        return out if stab > 0.0 else out[:4]   # no OSS operator without stabilisation
+
+    for call in (ppe, oss, system):
+        p.same(call)
