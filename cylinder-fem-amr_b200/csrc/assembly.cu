@@ -326,6 +326,20 @@ __global__ void k_oss_weights(int ne, const int* __restrict__ ev, const double* 
     elem_s[e] = rho * tau / dt;
 }
 
+// Area and grad f of one element (fem_kernels.cuh:735-752), rounded explicitly as the momentum's terms
+// are; false for a degenerate element. Its weight is gradient_weight.
+__device__ __forceinline__ bool gradient_element(double x0, double y0, double x1, double y1, double x2, double y2,
+                                                 double f0, double f1, double f2, double& area, double& gx,
+                                                 double& gy) {
+    area = 0.5 * fabs(__fma_rn(x1 - x0, y2 - y0, -__dmul_rn(x2 - x0, y1 - y0)));
+    if (area < 1.0e-14) return false;
+    const double inv2A = 1.0 / (2.0 * area);
+    gx = __dmul_rn(__fma_rn(f2, y0 - y1, __fma_rn(f0, y1 - y2, __dmul_rn(f1, y2 - y0))), inv2A);
+    gy = __dmul_rn(__fma_rn(f2, x1 - x0, __fma_rn(f0, x2 - x1, __dmul_rn(f1, x0 - x2))), inv2A);
+    return true;
+}
+__device__ __forceinline__ double gradient_weight(double rs, double area) { return __dmul_rn(rs, area) / 3.0; }
+
 // k_accumulate_scalar_gradient (fem_kernels.cuh:726-757), per row: G_i(f) numerators
 __global__ void k_scalar_gradient_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
                                        const double* __restrict__ y, const int* __restrict__ inc_ptr,
@@ -341,15 +355,11 @@ __global__ void k_scalar_gradient_rows(int n, const int* __restrict__ ev, const 
         int nd[3];
         load_elem(ev, e, nd);
         const double x0 = x[nd[0]], y0 = y[nd[0]], x1 = x[nd[1]], y1 = y[nd[1]], x2 = x[nd[2]], y2 = y[nd[2]];
-        const double detJ = (x1 - x0) * (y2 - y0) - (x2 - x0) * (y1 - y0);
-        const double area = 0.5 * fabs(detJ);
-        if (area < 1.0e-14) continue;
-        const double inv2A = 1.0 / (2.0 * area);
-        const double gx = (f[nd[0]] * (y1 - y2) + f[nd[1]] * (y2 - y0) + f[nd[2]] * (y0 - y1)) * inv2A;
-        const double gy = (f[nd[0]] * (x2 - x1) + f[nd[1]] * (x0 - x2) + f[nd[2]] * (x1 - x0)) * inv2A;
-        const double w = (elem_s ? sqrt(elem_s[e]) : 1.0) * area / 3.0;
-        sx += w * gx;
-        sy += w * gy;
+        double area, gx, gy;
+        if (!gradient_element(x0, y0, x1, y1, x2, y2, f[nd[0]], f[nd[1]], f[nd[2]], area, gx, gy)) continue;
+        const double w = gradient_weight(elem_s ? sqrt(elem_s[e]) : 1.0, area);
+        sx = __fma_rn(w, gx, sx);
+        sy = __fma_rn(w, gy, sy);
     }
     gx_out[i] = sx;
     gy_out[i] = sy;
@@ -530,16 +540,9 @@ k_scalar_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev, cons
         load_elem(ev, tv.elems[b.i0 + le], nd);
         const double es = elem_s ? elem_s[tv.elems[b.i0 + le]] : 1.0;
         const double x0 = x[nd[0]], y0 = y[nd[0]], x1 = x[nd[1]], y1 = y[nd[1]], x2 = x[nd[2]], y2 = y[nd[2]];
-        const double f0 = f[nd[0]], f1 = f[nd[1]], f2 = f[nd[2]];
-        const double detJ = (x1 - x0) * (y2 - y0) - (x2 - x0) * (y1 - y0);
-        const double area = 0.5 * fabs(detJ);
-        double gx = 0.0, gy = 0.0, w = 0.0;
-        if (!(area < 1.0e-14)) {
-            const double inv2A = 1.0 / (2.0 * area);
-            w = (elem_s ? sqrt(es) : 1.0) * area / 3.0;
-            gx = (f0 * (y1 - y2) + f1 * (y2 - y0) + f2 * (y0 - y1)) * inv2A;
-            gy = (f0 * (x2 - x1) + f1 * (x0 - x2) + f2 * (x1 - x0)) * inv2A;
-        }
+        double area, gx = 0.0, gy = 0.0, w = 0.0;
+        if (gradient_element(x0, y0, x1, y1, x2, y2, f[nd[0]], f[nd[1]], f[nd[2]], area, gx, gy))
+            w = gradient_weight(elem_s ? sqrt(es) : 1.0, area);
         et_rec[le] = gx;
         et_rec[S + le] = gy;
         et_rec[2 * S + le] = w;

@@ -265,3 +265,39 @@ def test_pressure_tiles_give_the_gathers_bits(name, stab):
 
     for call in (ppe, oss, system):
         p.same(call)
+
+
+@pytest.mark.parametrize("weighted", [True, False])
+@pytest.mark.parametrize("name", list(BIT_MESHES))
+def test_gradient_tiles_give_the_gathers_bits(name, weighted):
+    import cfa_b200 as cfa
+    p = _Pair(BIT_MESHES[name]())
+    m = p.m
+    f = [F.fourier_field(m.x, m.y, k) for k in range(1, 4)]
+    s = 0.5 + 0.4 * np.sin(np.arange(m.ne))
+
+    def scalar(dm, k):
+        q, es = p.fields(k, f[2], s)
+        out = [_empty(dm.n), _empty(dm.n)]
+        cfa.scalar_gradient(p.ctx, dm, q, es if weighted else None, *out)
+        return out
+
+    def node(dm, k):
+        u, v, dp = p.fields(k, *f)
+        out = [_empty(dm.n) for _ in range(3)]
+        cfa.grad_dp_vorticity(p.ctx, dm, dp, u, v, *out)
+        return out
+
+    def stiffness(dm, k):
+        out, dp = p.fields(k, f[0], f[2])
+        cfa.stiffness_apply(p.ctx, dm, dp, -0.37, out)
+        return [out]
+
+    def recovered(dm, k):
+        u, v, ms = p.fields(k, f[0], f[1], 1.0 + 0 * f[0])
+        rec = _empty(4 * dm.n)
+        cfa.amr_indicators(p.ctx, dm, u, v, 1.5, 1.0, ms, rec, _empty(2 * dm.ne))
+        return [rec]
+
+    for call in (scalar, node, stiffness, recovered):
+        p.same(call)
