@@ -3275,6 +3275,12 @@ int cfa_amg_remaps(const cfa_amg* amg) { return amg ? amg->remaps : 0; }
 cfa_status cfa_amg_apply(cfa_ctx* ctx, cfa_amg* amg, const double* r, double* z) {
     CFA_ENTER(ctx);
     CFA_ARG(amg && r && z && amg->coarse_n > 0);
+    if (r == z && amg_on_rings(amg)) {
+        // the last pair of sweeps reads b on a tile's ring while other blocks write z there
+        AmgLevel& L = amg->levels[0];
+        CFA_CUDA(cudaMemcpyAsync(L.ring.b.p, r, (size_t)L.A.rows * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+        r = L.ring.b.p;
+    }
     return amg_vcycle(ctx, amg, r, z, nullptr);
 }
 

@@ -232,6 +232,7 @@ cfa_status build_ring(cfa_ctx* ctx, int n, int nnz, const int* rp, const int* ci
     CFA_CUDA(R.ci.ensure(R.total + 8));
     if (f32) CFA_CUDA(R.v32.ensure(R.total + 8));
     if (f64) CFA_CUDA(R.v64.ensure(R.total + 8));
+    CFA_CUDA(R.b.ensure(n));
     CFA_LAUNCH(ctx, k_ring_fill, R.ntiles, kRingThreads, 0, n, R.rows, rp, ci, v, R.meta.p, (const int*)R.off.p,
                (const int*)R.halo.p, R.rp_stride, R.rp.p, R.ci.p, f32 ? R.v32.p : (float*)nullptr,
                f64 ? R.v64.p : (double*)nullptr);

@@ -36,6 +36,7 @@ struct RingTiles {
     DevBuf<unsigned short> ci;        // [total]
     DevBuf<float> v32;
     DevBuf<double> v64;
+    DevBuf<double> b;                 // [n]: the right-hand side of an apply in place
     DevBuf<int> cnt;                  // planning: padded entries per tile, then their offsets
     DevBuf<int> off, flags;
     DevBuf<unsigned char> tmp;

@@ -412,7 +412,8 @@ cfa_status cfa_amg_remap(cfa_ctx* ctx, cfa_amg* amg, int n, int nnz, const int* 
                          const int* h_col_ind, const int* h_new_to_old);
 /* remaps: remap() calls that reused the hierarchy (the reference's `remaps`). */
 int cfa_amg_remaps(const cfa_amg* amg);
-/* apply (:1161-1168): one symmetric V-cycle, z = M^-1 r. */
+/* apply (:1161-1168): one symmetric V-cycle, z = M^-1 r. d_z may be d_r on a hierarchy of two or more
+ * levels; otherwise the arrays must not overlap. */
 cfa_status cfa_amg_apply(cfa_ctx* ctx, cfa_amg* amg, const double* d_r, double* d_z);
 /* num_levels() (reference: levels with P + the coarsest), coarse_n, setup time [ms] */
 cfa_status cfa_amg_info(const cfa_amg* amg, int* num_levels, int* coarse_n, double* setup_ms);

@@ -97,3 +97,28 @@ def test_cg_update_in_the_ring_kernel(precision, monkeypatch):
         # a solve to 1e-10 at its tolerance
         lim = 1e-11 if precision == "fp64" and i1 <= 6 else 1e-5 if i1 <= 40 else 1e-7
         assert float((x0 - x1).norm()) <= lim * float(x1.norm()), (k, i0, i1)
+
+
+@pytest.mark.parametrize("name", list(MESHES))
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_apply_in_place(name, precision):
+    import torch
+    import cfa_b200 as cfa
+    m = MESHES[name]()
+    ctx = cfa.default_context()
+    dm = cfa.DeviceMesh(ctx, m)
+    n, nnz = dm.n, dm.nnz
+    z = lambda k: torch.zeros(k, dtype=torch.float64, device="cuda")
+    K, rhs, div, dp, g, mass = z(nnz), z(n), z(n), z(n), z(n), z(n)
+    t = lambda a: torch.from_numpy(a).to("cuda")
+    u, v = t(F.fourier_field(m.x, m.y, 1)), t(F.fourier_field(m.x, m.y, 2))
+    cfa.assemble_ppe(ctx, dm, u, v, z(n), g, g, mass, z(m.ne), 1e-3, 1.0, 0.0, K, rhs, div, dp)
+    amg = cfa.AmgPreconditioner(ctx, cfa.MIXED if precision == "mixed" else cfa.FP64)
+    amg.setup(n, nnz, dm.rp, dm.ci, K)
+    assert amg.num_levels() > 1
+    want = z(n)
+    amg.apply(rhs, want)
+    for _ in range(5):
+        x = rhs.clone()
+        amg.apply(x, x)
+        assert torch.equal(x, want)
