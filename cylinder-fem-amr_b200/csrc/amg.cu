@@ -1166,14 +1166,14 @@ static void vct(cfa_ctx* ctx, bool dry, const TiledCsr& M, int* err, const T* di
 // ---------------------------------------------------------------------------------------------
 // level 0's sweeps in pairs over ring tiles (ring.cuh)
 // ---------------------------------------------------------------------------------------------
-// RING_PRE: x = VC_PRE of b, out = b - A x; RING_PREC: the same with the first iterate c = x given;
-// RING_JAC: out = two Jacobi sweeps from x (RZ: with the CG's dots of out). xout: RING_PRE(C)'s x.
+// RING_PRE: x = VC_PRE of b, out = b - A x;
+// RING_JAC: out = two Jacobi sweeps from x (RZ: with the CG's dots of out). xout: RING_PRE's x.
 // RING_CGU: RING_PRE of the residual r - alpha q after the CG's update, which it also does on its own
 // rows (k_cg_update's operations), with |r| and the stopping test.
 // Bound by latency at the sizes that take it (ring_rows, ring.cu): one round of gathers, then two
 // sweeps from shared memory, in place of two kernels. 8k vertices: a pair of kernels 7.4 us -> 4.1 us,
 // the FP64 V-cycle 28.7 -> 21.0 us; 37k: 35.2 -> 31.7 us.
-enum RingOp { RING_PRE = 0, RING_PREC = 1, RING_JAC = 2, RING_CGU = 3 };
+enum RingOp { RING_PRE = 0, RING_JAC = 1, RING_CGU = 2 };
 
 // One row's sum over its entries in order, the loads of a batch ahead of its sums
 template <class V, class T>
@@ -1744,14 +1744,13 @@ static void vcycle_tiled(cfa_ctx* ctx, cfa_amg* amg, int l, const B* b, double* 
     const T* dinv = TVec<T>::dinv(L);
     T* x = TVec<T>::x(L);
     T* t = TVec<T>::t(L);
-    const bool ring = L.ring.ok;   // level 0, two smoothing steps: sweeps in pairs
+    // level 0, two smoothing steps: sweeps in pairs (they take the CG's update, so no c0: amg_can_fuse_update)
+    const bool ring = L.ring.ok;
     if (ring) {
-        if ((c0 && !cg) || dry)
-            ring_sweeps<RING_PREC, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, c0, x, TVec<T>::r(L), done, rz);
         if (cg || dry)
             ring_sweeps<RING_CGU, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, (const T*)nullptr, x,
                                               TVec<T>::r(L), done, rz, cg);
-        if ((!c0 && !cg) || dry)
+        if (!cg || dry)
             ring_sweeps<RING_PRE, V, T, B, T>(ctx, dry, L.ring, err, dinv, omega, b, (const T*)nullptr, x,
                                               TVec<T>::r(L), done, rz);
     } else if (s >= 2 && c0 && !cg) {   // the first iterate formed by the caller
