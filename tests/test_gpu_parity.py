@@ -26,7 +26,12 @@ MESHES = {}
 
 def mesh(name):
     if name not in MESHES:
-        MESHES[name] = F.make_mesh(name)
+        if name == "113k":   # level 0 beyond the ring tiles (512 rows per SM)
+            import batch as B
+            MESHES[name] = B.batch_system(3, 77_001, 77_001).mesh
+            assert MESHES[name].n > 512 * torch.cuda.get_device_properties(0).multi_processor_count
+        else:
+            MESHES[name] = F.make_mesh(name)
     return MESHES[name]
 
 
@@ -684,14 +689,16 @@ def test_pcg_matches_oracle(ctx, use_oss, use_amg):
     assert np.linalg.norm(rhs - Ax) <= 1.5e-10 * np.linalg.norm(rhs)
 
 
+@pytest.mark.parametrize("name", ["c0", "113k"])
 @pytest.mark.parametrize("prec", [cfa.FP64, cfa.MIXED])
-def test_pcg_update_folded_into_vcycle_matches_update_kernel(ctx, prec, monkeypatch):
+def test_pcg_update_folded_into_vcycle_matches_update_kernel(ctx, name, prec, monkeypatch):
     """The CG's update (x += alpha pn, r -= alpha q, p = pn, |r| and the stopping test) folded into
     the V-cycle's level-0 pre-smoothing and residual passes, against the separate update kernel:
     the same arithmetic per row (up to where the compiler contracts the update into a fused
     multiply-add), so iteration counts within 1, solutions within 1e-8, and the true residual of
-    the folded solve below 1.5e-10."""
-    m = mesh("c0")
+    the folded solve below 1.5e-10. (By default c0 folds it into the ring tiles' kernel, the larger
+    mesh runs the update kernel.)"""
+    m = mesh(name)
     dm = cfa.DeviceMesh(ctx, m)
     rp, ci = dm.host_pattern()
     Kp, rhs, oss, inv_m = pressure_system(m, rp, ci)
@@ -714,12 +721,13 @@ def test_pcg_update_folded_into_vcycle_matches_update_kernel(ctx, prec, monkeypa
     assert np.linalg.norm(rhs - Ax) <= 1.5e-10 * np.linalg.norm(rhs)
 
 
+@pytest.mark.parametrize("name", ["c0", "113k"])
 @pytest.mark.parametrize("prec", [cfa.FP64, cfa.MIXED])
-def test_pcg_prescaled_residual_gives_the_same_bits(ctx, prec, monkeypatch):
+def test_pcg_prescaled_residual_gives_the_same_bits(ctx, name, prec, monkeypatch):
     """The CG update writing c = omega0 D0^-1 r (in the V-cycle's vector type) for the level-0
     pre-smoothing, which then gathers c instead of D0^-1 and r: the products are formed in the
     same order, so the solve is bit-identical to the one that forms them inside the V-cycle."""
-    m = mesh("c0")
+    m = mesh(name)
     dm = cfa.DeviceMesh(ctx, m)
     rp, ci = dm.host_pattern()
     Kp, rhs, oss, inv_m = pressure_system(m, rp, ci)

@@ -25,9 +25,28 @@ MESHES = {
     "small": lambda: F.make_mesh("small"),
     "small_shuffled": lambda: _shuffled(F.make_mesh("small")),
     "c0": lambda: F.make_mesh("c0"),
-    "60k": lambda: _target(60_001),
+    "64k": lambda: _target(60_000, 3),
+    "76k": lambda: _target(60_001, 5),     # 75,972 vertices, just above 512 rows per SM
+    "100k": lambda: _target(60_001),
     "160k": lambda: _target(160_001),
 }
+
+
+# Whether level 0 takes ring tiles: not where a tile's rings do not fit (a random numbering of more than
+# a few thousand vertices), nor above 512 rows per SM
+ON_RINGS = {"small": True, "small_shuffled": False, "c0": True,
+            "64k": True, "76k": False, "100k": False, "160k": False}
+
+
+def _kernels(call):
+    """Names of the kernels that `call` launches outside a graph."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events() if "k_" in e.name]
 
 
 @pytest.mark.parametrize("name", list(MESHES))
@@ -54,6 +73,9 @@ def test_vcycle_bits(name, precision, monkeypatch):
         amg.apply(out.clone(), out)
         torch.cuda.synchronize()
         assert torch.isfinite(out).all() and float(out.abs().max()) > 0.0
+        names = _kernels(lambda: amg.apply(rhs, z(n)))
+        assert any("k_vct" in k for k in names)
+        assert any("k_ring" in k for k in names) == (fused == "0" and ON_RINGS[name]), names
         got.append(out)
     assert torch.equal(got[0], got[1])
 
