@@ -2105,11 +2105,27 @@ __global__ void k_agg_p2(int n, const int* __restrict__ rp, const int* __restric
 // 3 together at 402k vertices 6.36 -> 6.21 ms, at 43k 2.21 -> 1.75 ms).
 // Progress: the lowest undecided node has all its lower conflicts decided, and its chunk has
 // started, because every CTA with an earlier ticket holds only lower nodes, all decided, and
-// retires. Every wait is bounded: a thread that polls kAggPollLimit times, or sees another thread
-// give up, records CFA_TIMEOUT in *err and leaves its node undecided.
+// retires. Every wait is bounded in time, looked at every kAggCheck polls: a thread that has waited
+// limit_ns, or sees another thread give up, records CFA_TIMEOUT in *err and leaves its node undecided.
+// The longest wait that can resolve is a chain through all resident chunks (a path graph in its natural
+// order: 2 x 148 x 1024 nodes at 0.9 us each, 0.27 s); kAggWaitNs is seven times that.
 constexpr int kAggChunk = 1024;
 constexpr int kAggBatch = 16;
-constexpr unsigned kAggPollLimit = 1u << 25;
+constexpr unsigned kAggCheck = 64;
+constexpr unsigned long long kAggWaitNs = 2'000'000'000ull;
+
+// CFA_AGG_WAIT_MS in the environment overrides the limit
+static unsigned long long agg_wait_ns() {
+    const char* e = std::getenv("CFA_AGG_WAIT_MS");
+    if (!e || !*e) return kAggWaitNs;
+    const double ms = std::atof(e);
+    return ms >= 0.0 && ms <= 1e4 ? (unsigned long long)(ms * 1e6) : kAggWaitNs;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
 
 struct AggView {
     const unsigned char* g;     // global states
@@ -2180,7 +2196,7 @@ __device__ __forceinline__ unsigned char agg_decide(int i, const int* __restrict
 template <bool P3>
 __global__ void __launch_bounds__(kAggChunk)
 k_agg_flow(int n, const int* __restrict__ lptr, const int* __restrict__ list, unsigned char* st,
-           int* __restrict__ ticket, int* err) {
+           int* __restrict__ ticket, int* err, unsigned long long limit_ns) {
     CFA_GRID_DEP();
     __shared__ int s_chunk;
     __shared__ unsigned char s_st[kAggChunk];
@@ -2196,6 +2212,7 @@ k_agg_flow(int n, const int* __restrict__ lptr, const int* __restrict__ list, un
     const int beg = i < n ? lptr[i] : 0, end = i < n ? lptr[i + 1] : 0;
     constexpr int kMask = 64;   // list entries under the mask; longer lists look at the rest last
     unsigned long long pend = end - beg >= kMask ? ~0ull : (1ull << (end - beg)) - 1ull;
+    unsigned long long since = 0;   // the first check's time
     for (unsigned it = 0; mine == AGG_UNDECIDED; ++it) {
         bool root = false;
         for (unsigned long long p = pend; p != 0ull && !root;) {
@@ -2223,9 +2240,13 @@ k_agg_flow(int n, const int* __restrict__ lptr, const int* __restrict__ list, un
         if (mine != AGG_UNDECIDED) {
             s_st[threadIdx.x] = mine;
             *reinterpret_cast<volatile unsigned char*>(st + i) = mine;
-        } else if (it >= kAggPollLimit || ((it & 63u) == 63u && *verr != 0)) {
-            atomicCAS(err, 0, (int)CFA_TIMEOUT);
-            break;
+        } else if (it % kAggCheck == kAggCheck - 1) {
+            const unsigned long long now = global_ns();
+            if (since == 0) since = now;
+            if (now - since >= limit_ns || *verr != 0) {
+                atomicCAS(err, 0, (int)CFA_TIMEOUT);
+                break;
+            }
         }
     }
 }
@@ -2319,7 +2340,7 @@ static cfa_status aggregate_device(cfa_ctx* ctx, SetupScratch& S, const DCsr& A,
     CFA_CUDA(cudaMemsetAsync(S.ag_state.p, AGG_UNDECIDED, n, ctx->stream));
     CFA_CUDA(cudaMemsetAsync(S.ag_flag.p, 0, 2 * sizeof(int), ctx->stream));
     CFA_LAUNCH(ctx, k_agg_flow<false>, chunks, kAggChunk, 0, n, (const int*)S.ag_cptr.p, (const int*)S.ag_conf.p,
-               S.ag_state.p, S.ag_flag.p, S.ag_flag.p + 1);
+               S.ag_state.p, S.ag_flag.p, S.ag_flag.p + 1, agg_wait_ns());
     CFA_LAUNCH(ctx, k_agg_is_root, g1, kThreads, 0, n, (const unsigned char*)S.ag_state.p, S.ag_fill.p);
     CFA_PROPAGATE(exclusive_sum(ctx, S, S.ag_fill.p, S.ag_rank.p, n));
     CFA_LAUNCH(ctx, k_agg_p1_ids, g, kThreads, 0, n, (const int*)S.ag_trp.p, (const int*)S.ag_tci.p,
@@ -2331,11 +2352,11 @@ static cfa_status aggregate_device(cfa_ctx* ctx, SetupScratch& S, const DCsr& A,
     CFA_CUDA(cudaMemcpyAsync(S.h_ag.p + 1, S.ag_rank.p + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CFA_CUDA(cudaMemsetAsync(S.ag_flag.p, 0, sizeof(int), ctx->stream));
     CFA_LAUNCH(ctx, k_agg_flow<true>, chunks, kAggChunk, 0, n, (const int*)S.ag_trp.p, (const int*)S.ag_tci.p,
-               S.ag_state.p, S.ag_flag.p, S.ag_flag.p + 1);
+               S.ag_state.p, S.ag_flag.p, S.ag_flag.p + 1, agg_wait_ns());
     CFA_CUDA(cudaMemcpyAsync(S.h_ag.p + 2, S.ag_flag.p + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CFA_CUDA(cudaStreamSynchronize(ctx->stream));
     if (S.h_ag.p[2] != 0)
-        return set_error(ctx, CFA_TIMEOUT, "aggregation: a node's decision waited past its poll limit", __FILE__,
+        return set_error(ctx, CFA_TIMEOUT, "aggregation: a node's decision waited past its limit", __FILE__,
                          __LINE__);
     const int na1 = S.h_ag.p[1];
     CFA_LAUNCH(ctx, k_agg_is_root, g1, kThreads, 0, n, (const unsigned char*)S.ag_state.p, S.ag_fill.p);

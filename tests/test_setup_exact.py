@@ -76,3 +76,26 @@ def test_hierarchy_bits(name, monkeypatch):
                 assert np.array_equal(got[k][0].cpu().numpy(), orp), (lv, k)
                 assert np.array_equal(got[k][1].cpu().numpy(), oci), (lv, k)
                 assert np.array_equal(got[k][2].cpu().numpy(), ov), (lv, k)
+
+
+def test_aggregation_wait_runs_out(monkeypatch):
+    """A path graph in its natural order decides node after node. With no time allowed the waiting threads
+    give up, the setup reports it, and the same handle sets the same matrix up afterwards."""
+    import torch
+    import cfa_b200 as cfa
+    from oracle import oracle as O
+    n = 20_000
+    rows = [{j: -1.0 for j in (i - 1, i + 1) if 0 <= j < n} | {i: 2.001} for i in range(n)]
+    rp, ci, v = _csr(rows)
+    t = lambda a: torch.from_numpy(a).to("cuda")
+    d = (t(rp), t(ci), t(v))
+    amg = cfa.AmgPreconditioner(cfa.default_context())
+    amg.set_aggregation(1)
+    monkeypatch.setenv("CFA_AGG_WAIT_MS", "0")
+    with pytest.raises(cfa.CfaError) as e:
+        amg.setup(n, len(ci), *d)
+    assert e.value.status == cfa.CFA_TIMEOUT
+    monkeypatch.delenv("CFA_AGG_WAIT_MS")
+    amg.setup(n, len(ci), *d)
+    want = O.Amg(rp, ci, v).level(0)
+    assert np.array_equal(amg.level(0)["agg"].cpu().numpy(), want["agg"])
