@@ -232,17 +232,43 @@ k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __rest
     }
     __syncthreads();
     // row by row: an entry's contributions are the (incidence, column) pairs whose position it is
+    auto code = [&](int s, int b) { return (unsigned short)(((rc[s] >> 2) << 4) | ((rc[s] & 3) << 2) | b); };
     for (int i = r0 + threadIdx.x; i < r1; i += kEtThreads) {
         const int s0 = inc_ptr[i] - i0, s1 = inc_ptr[i + 1] - i0;
+        if (s1 - s0 > kEtLongRow) continue;
         int cur = 3 * s0;
         for (int p = rp[i]; p < rp[i + 1]; ++p) {
             eoff[p] = (unsigned short)cur;
             for (int s = s0; s < s1; ++s)
 #pragma unroll
                 for (int b = 0; b < 3; ++b)
-                    if (pos[3 * (size_t)(i0 + s) + b] == p)
-                        ecode[3 * (size_t)i0 + cur++] =
-                            (unsigned short)(((rc[s] >> 2) << 4) | ((rc[s] & 3) << 2) | b);
+                    if (pos[3 * (size_t)(i0 + s) + b] == p) ecode[3 * (size_t)i0 + cur++] = code(s, b);
+        }
+    }
+    // a row of many elements by the whole block, an entry per thread: its contributions counted, their
+    // offsets from a scan, then written (one thread would look through all pairs for every entry)
+    for (int i = r0; i < r1; ++i) {
+        const int s0 = inc_ptr[i] - i0, s1 = inc_ptr[i + 1] - i0;
+        if (s1 - s0 <= kEtLongRow) continue;   // the same for all threads
+        const int* ps = pos + 3 * (size_t)(i0 + s0);
+        int carry = 3 * s0;
+        for (int p0 = rp[i]; p0 < rp[i + 1]; p0 += kEtThreads) {
+            const int p = p0 + threadIdx.x, pairs = 3 * (s1 - s0);
+            const bool has = p < rp[i + 1];
+            int count = 0, before = 0, sum = 0;
+            if (has)
+#pragma unroll 8
+                for (int k = 0; k < pairs; ++k) count += ps[k] == p;
+            __syncthreads();
+            Scan(tmp.scan).ExclusiveSum(count, before, sum);
+            if (has) {
+                int cur = carry + before;
+                eoff[p] = (unsigned short)cur;
+#pragma unroll 8
+                for (int k = 0; k < pairs; ++k)
+                    if (ps[k] == p) ecode[3 * (size_t)i0 + cur++] = code(s0 + k / 3, k % 3);
+            }
+            carry += sum;
         }
     }
 }

@@ -18,6 +18,7 @@ namespace cfa {
 constexpr int kEtThreads = 256;
 constexpr int kEtRows = 96;                    // rows of a tile
 constexpr int kEtMaxInc = 12 * kEtThreads;     // incidences of a tile that the plan can sort
+constexpr int kEtLongRow = 24;                  // incidences of a row that one thread of the plan takes
 constexpr int kEtMaxSmem = 200 * 1024;         // bytes of shared memory a tile may need
 constexpr int kEtMaxRec = 19;                  // doubles per element of the largest records
 

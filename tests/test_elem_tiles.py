@@ -43,7 +43,11 @@ CASES = {
     "small_shuffled": lambda: _shuffled(F.make_mesh("small")),
     "c0_rows64": lambda: F.make_mesh("c0"),
     "medium_rows96": lambda: F.make_mesh("medium"),
+    "wheel_24": lambda: _wheel(24),              # one thread plans the row
+    "wheel_25": lambda: _wheel(25),              # the whole block does
     "wheel_127": lambda: _wheel(127),
+    "wheel_255": lambda: _wheel(255),            # 256 entries in the row, as many as threads
+    "wheel_256": lambda: _wheel(256),
     "wheel_1200": lambda: _wheel(1200),          # one tile with nearly all of a block's shared memory
     "wheel_2000_gather": lambda: _wheel(2000),   # records beyond it: the row gathers
     "wheel_3100_gather": lambda: _wheel(3100),   # incidences beyond the plan's sort
