@@ -197,7 +197,11 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
 // and square roots of the element formula, then the entries' codes. Against the row gather: 142 ->
 // 130 us at 402k vertices (130 MB, 1.0 TB/s), 21.0 -> 13.3 us at 22.5k, 19.5 -> 13.2 us at 8k.
 // Three blocks per SM (80 registers) matter: at 92 registers, two blocks, 189 against 144 us at 402k
-// vertices, each with the L2 flushed first.
+// vertices, each with the L2 flushed first. A wave of tiles (3 x 148 of 96 rows) takes some 14 us, one of
+// gathers (2 x 148 of 256 rows) some 24, so tiles run up to 5/3 of the gathers' waves. Tiles / gathers in
+// us: 37k vertices 26 / 28, 56k 36 / 34, 76k 38 / 45, 113k 50 / 57, 135k 61 / 58, 156k 65 / 73, 317k
+// 118 / 123, 402k 144 / 149, 642k 220 / 221, 1.3M 427 / 419, 4.2M 1350 / 1317.
+constexpr EtForm kMomForm = {3, 2, 5, 3};
 __global__ void __launch_bounds__(kEtThreads, 3)
 k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
                  const double* __restrict__ y, const int* __restrict__ tag, const int* __restrict__ rp,
@@ -522,10 +526,10 @@ k_pressure_rows(int n, int nnz, const int* __restrict__ ev, const double* __rest
 }
 
 // Scalar gradient on element tiles: grad f and the weight (area / 3) sqrt(s) of every element
-// once, then the rows. Against the row gather 9.4 -> 6.3 us at 22.5k vertices, 8.3 -> 6.1 us at 8k,
-// 29.9 -> 31.0 us at 402k, 269 -> 389 us at 4.2M: the tile's plan is as many bytes as it saves, so
-// the form pays only while the mesh is latency (kGradTileRows).
-constexpr int kGradTileRows = 150'000;
+// once, then the rows. The tile's plan is as many bytes as it saves, so the form pays while it is one
+// wave (5 blocks of 96 rows an SM, 71k vertices). Tiles / gathers in us, the L2 flushed first: 7k vertices
+// 10.2 / 18.5, 22k 10.3 / 18.0, 66k 14.3 / 18.6, 76k 18.4 / 18.4, 100k 20.5 / 19.5, 135k 22.3 / 20.5.
+constexpr EtForm kGradForm = {5, 5, 1, 1};
 
 __global__ void __launch_bounds__(kEtThreads)
 k_scalar_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
@@ -753,7 +757,7 @@ cfa_status cfa_assemble_momentum_nu(cfa_ctx* ctx, const cfa_mesh* m, const doubl
     MomParams P{prm->dt, prm->nu, prm->rho, prm->a0, prm->a1, prm->a2, prm->c1, prm->c2, prm->tau_time, prm->skew_coef};
     const double u_max = bcp ? bcp->u_max : 0.0, H = bcp ? bcp->H : 1.0;
     allow_et_kernels();
-    if (m->et.ok)
+    if (et_better(m->et, m->n, ctx->num_sms, kMomForm))
         CFA_LAUNCH(ctx, k_momentum_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 16), m->tiles(), m->n, m->ev,
                    m->x, m->y, m->tag, m->rp, m->ci, u_old, v_old, u_prev, v_prev, p_old, nu_node, P, bcp ? 1 : 0, u_max, H, m->bc,
                    A_val, rhs_u, rhs_v, mass);
@@ -802,7 +806,7 @@ cfa_status cfa_scalar_gradient(cfa_ctx* ctx, const cfa_mesh* m, const double* f,
     CFA_ENTER(ctx);
     CFA_ARG(m && f && gx && gy);
     allow_et_kernels();
-    if (m->et.ok && m->n <= kGradTileRows)
+    if (et_better(m->et, m->n, ctx->num_sms, kGradForm))
         CFA_LAUNCH(ctx, k_scalar_gradient_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 3), m->tiles(), m->n,
                    m->ev, m->x, m->y, f, elem_s, gx, gy);
     else

@@ -166,7 +166,8 @@ static cfa_status build_incidence(cfa_ctx* ctx, int n, int ne, const int* d_ev, 
 
 // Element tiles (elemtile.cuh), one block per tile: its incidences' elements sorted and made unique,
 // the local element of every incidence, and every CSR entry's contributions in incidence order.
-// flags[0]: the largest element count, flags[1]: a tile with too many incidences.
+// flags[0]: the largest element count, [1]: a tile with too many incidences, [2]: the sum of the element
+// counts, [3]: most elements around one vertex.
 __global__ void __launch_bounds__(kEtThreads)
 k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __restrict__ inc,
              const int* __restrict__ pos, const int* __restrict__ rp, int* __restrict__ elems,
@@ -184,6 +185,10 @@ k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __rest
     __shared__ unsigned short rc[kEtMaxInc];
     CFA_GRID_DEP();   // pos is the kernel before's output
     const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+    int longest = 0;
+    for (int i = r0 + threadIdx.x; i < r1; i += kEtThreads) longest = max(longest, inc_ptr[i + 1] - inc_ptr[i]);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0 && longest > kEtHubRow) atomicMax(&flags[3], longest);
     const int i0 = inc_ptr[r0], m = inc_ptr[r1] - i0;
     if (m > kEtMaxInc) {
         if (threadIdx.x == 0) {
@@ -217,6 +222,7 @@ k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __rest
     if (threadIdx.x == 0) {
         count[blockIdx.x] = total;
         atomicMax(&flags[0], total);
+        atomicAdd(&flags[2], total);
     }
     __syncthreads();
     for (int s = threadIdx.x; s < m; s += kEtThreads) {
@@ -273,7 +279,7 @@ k_elem_tiles(int n, int rows, const int* __restrict__ inc_ptr, const int* __rest
     }
 }
 
-// The mesh's element tiles; flags (2 ints, zeroed) are read back by the caller.
+// The mesh's element tiles; flags (4 ints, zeroed) are read back by the caller.
 static cudaError_t plan_elem_tiles(cfa_ctx* ctx, cfa_mesh* m, int nnz, int* flags) {
     ElemTiles& T = m->et;
     T.rows = elem_tile_rows(m->n, ctx->num_sms);
@@ -446,8 +452,8 @@ cfa_status cfa_mesh_create(cfa_ctx* ctx, int n, int ne, const int* d_ev, const d
     DevBuf<int> err;   // a missing entry, then the element tiles' flags
     int h_nnz = 0;
     cudaError_t e = m->pos.ensure(9 * (size_t)ne);
-    if (e == cudaSuccess) e = err.ensure(3);
-    if (e == cudaSuccess) e = cudaMemsetAsync(err.p, 0, 3 * sizeof(int), ctx->stream);
+    if (e == cudaSuccess) e = err.ensure(5);
+    if (e == cudaSuccess) e = cudaMemsetAsync(err.p, 0, 5 * sizeof(int), ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_nnz, d_rp + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) { delete m; return set_error(ctx, CFA_CUDA_ERROR, cudaGetErrorString(e), __FILE__, __LINE__); }
@@ -455,13 +461,21 @@ cfa_status cfa_mesh_create(cfa_ctx* ctx, int n, int ne, const int* d_ev, const d
     k_scatter_positions<<<ceil_div(n, kThreads), kThreads, 0, ctx->stream>>>(n, d_ev, m->inc_ptr.p, m->inc.p, d_rp,
                                                                                d_ci, m->pos.p, err.p);
     e = plan_elem_tiles(ctx, m, h_nnz, err.p + 1);
-    int h_err[3] = {0, 0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_err, err.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    int h_err[5] = {0, 0, 0, 0, 0};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_err, err.p, 5 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) { delete m; return set_error(ctx, CFA_CUDA_ERROR, cudaGetErrorString(e), __FILE__, __LINE__); }
     if (h_err[0]) { delete m; return set_error(ctx, CFA_BAD_ARG, "element edge missing from the CSR pattern", __FILE__, __LINE__); }
-    m->et.max_elems = (h_err[1] + 3) & ~3;
-    m->et.ok = !h_err[2] && et_smem_bytes(m->et, kEtMaxRec) <= kEtMaxSmem;
+    ElemTiles& et = m->et;
+    et.max_elems = (h_err[1] + 3) & ~3;
+    et.repeats = (double)h_err[3] / ne;
+    et.max_row = h_err[4];
+    et.ok = !h_err[2] && et_smem_bytes(et, kEtMaxRec) <= kEtMaxSmem &&
+            (et.rows < kEtRows || et.repeats <= kEtRepeatsPressure);
+    if (!et.ok) {
+        for (DevBuf<int>* b : {&et.elems, &et.count}) b->release();
+        for (DevBuf<unsigned short>* b : {&et.rcode, &et.ecode, &et.eoff}) b->release();
+    }
     m->nnz = h_nnz;
     *out = m;
     return CFA_OK;

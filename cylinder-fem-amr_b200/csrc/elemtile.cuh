@@ -8,7 +8,8 @@
 // sum from there, in ascending element order as the gathers do, so the sums keep their order.
 //
 // The plan is connectivity only (made with the mesh handle); coordinates and fields are read at
-// every call.
+// every call. It takes 43 bytes an element (65 as the buffers are sized), beside 56 of the handle's
+// incidences and positions; a mesh whose kernels all take the row gathers gives it back.
 #pragma once
 
 #include "internal.cuh"
@@ -21,12 +22,21 @@ constexpr int kEtMaxInc = 12 * kEtThreads;     // incidences of a tile that the 
 constexpr int kEtLongRow = 24;                  // incidences of a row that one thread of the plan takes
 constexpr int kEtMaxSmem = 200 * 1024;         // bytes of shared memory a tile may need
 constexpr int kEtMaxRec = 19;                  // doubles per element of the largest records
+// Elements of all tiles over elements of the mesh (ElemTiles::repeats): 1.42 in the mesh's own order, 1.9
+// in reverse Cuthill-McKee's, 2.1 to 2.8 sorted by x, 3 (nothing shared) in a random one. Tiles against
+// gathers in us: sorted by x, 402k vertices: momentum 239 / 169, pressure 303 / 396, projection 105 / 89;
+// Cuthill-McKee: 153 / 153, 185 / 370, 67 / 75; random, 37k: 48 / 36, 60 / 51, 42 / 28, and pressure at
+// 4.2M 13.96 / 9.89 ms. Small meshes (64-row tiles) gain in any order: random, 22k: 29 / 36, 41 / 51, 24 / 28.
+constexpr double kEtRepeats = 2.0;             // most that the momentum and gradient kernels take
+constexpr double kEtRepeatsPressure = 2.9;     // ... the pressure's, and with it any
 
 struct ElemTiles {
-    bool ok = false;          // false: some tile is too large, the row gathers run instead
+    bool ok = false;          // false: the row gathers run instead (a tile too large, elements hardly shared)
     int rows = 0;             // rows per tile
     int ntiles = 0;
     int max_elems = 0;        // largest tile's element count, rounded up to a multiple of 4
+    int max_row = 0;          // most elements around one vertex
+    double repeats = 0.0;     // elements of all tiles / elements of the mesh
     DevBuf<int> elems;        // [3 ne]: tile t's elements ascending, from inc_ptr[first row]
     DevBuf<int> count;        // [ntiles]
     DevBuf<unsigned short> rcode;   // [3 ne]: incidence s -> local element << 2 | local vertex
@@ -47,6 +57,22 @@ struct ElemTileView {
 // feel first. Meshes with fewer than two such tiles per SM take 64 rows (22.5k vertices: 13.3 / 10.8
 // against 13.3 / 13.3 us).
 inline int elem_tile_rows(int n, int num_sms) { return n < 2 * num_sms * kEtRows ? 64 : kEtRows; }
+
+// Whether a kernel's tiles are its better form on this mesh. Both forms take whole waves of blocks, and
+// a wave of tiles costs a share of a wave of gathers that the kernel's comment states: tile_blocks and
+// row_blocks are the blocks an SM holds of each, num / den the most waves of tiles per wave of gathers.
+// A gather runs a long row in one thread (0.25 to 1.1 us an element), which tiles share.
+struct EtForm {
+    int tile_blocks, row_blocks, num, den;
+};
+constexpr int kEtHubRow = 31;
+inline bool et_better(const ElemTiles& t, int n, int num_sms, const EtForm& f) {
+    if (!t.ok || (t.rows == kEtRows && t.repeats > kEtRepeats)) return false;
+    if (t.max_row > kEtHubRow) return true;
+    const long long tiles = ceil_div(t.ntiles, f.tile_blocks * num_sms);
+    const long long gathers = ceil_div(ceil_div(n, kThreads), f.row_blocks * num_sms);
+    return tiles * f.den <= gathers * f.num;
+}
 
 // One tile of this block: rows [r0, r1), incidences [i0, i1), ne elements.
 struct EtBlock {

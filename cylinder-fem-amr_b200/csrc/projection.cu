@@ -73,7 +73,16 @@ k_node_gradients(int n, const int* __restrict__ ev, const double* __restrict__ x
 }
 
 // k_node_gradients on element tiles (elemtile.cuh): the element's six values once, then the nodes.
-// Bound by latency (elemtile.cuh): 27.9 -> 17.3 us at 120k vertices; the recovered gradient 23.1 -> 15.5 us.
+// Bound by latency, from a million vertices by HBM. With everything asked for (project_step, correction
+// included) tiles are the better form at every size: tiles / gathers in us, the L2 flushed first, 22k
+// vertices 17 / 22, 156k 34 / 42, 402k 60 / 72, 1.3M 181 / 194, 4.2M 556 / 577. With grad dp and the
+// vorticity alone, or the stiffness alone, a wave of tiles (5 x 148 of 96 rows) is half a wave of gathers
+// (4 x 148 of 256): 22k 12 / 17, 66k 14 / 19, 135k 21 / 21, 156k 26 / 31, 402k 47 / 49, 642k 74 / 74,
+// 1.3M 137 / 127, 4.2M 414 / 371; the stiffness 12 / 16, 14 / 19, 21 / 23, 25 / 29, 43 / 49, 68 / 72,
+// 127 / 126, 375 / 369.
+constexpr EtForm kNodeForm = {5, 4, 2, 1};
+constexpr EtForm kNodeAllForm = {1, 1, 1 << 20, 1};   // any number of waves
+
 __global__ void __launch_bounds__(kEtThreads)
 k_node_gradients_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
                        const double* __restrict__ y, const double* __restrict__ f, double c,
@@ -148,7 +157,7 @@ static cfa_status node_gradients(cfa_ctx* ctx, const cfa_mesh* m, const double* 
                                  const double* dp, const double* u, const double* v, double* gdx, double* gdy,
                                  double* vort_num) {
     allow_post_kernels();
-    if (m->et.ok)
+    if (et_better(m->et, m->n, ctx->num_sms, stiff && gdx ? kNodeAllForm : kNodeForm))
         CFA_LAUNCH(ctx, k_node_gradients_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 8), m->tiles(), m->n, m->ev, m->x,
                    m->y, f, c, stiff, dp, u, v, gdx, gdy, vort_num);
     else
@@ -270,7 +279,11 @@ k_recovered_gradient(int n, const int* __restrict__ ev, const double* __restrict
     for (int c = 0; c < 4; ++c) grad_rec[(size_t)c * n + i] = s[c];
 }
 
-// k_recovered_gradient on element tiles
+// k_recovered_gradient on element tiles, 4 blocks an SM in either form. Tiles / gathers in us, indicators
+// included, the L2 flushed first: 22k vertices 15 / 22, 56k 17 / 25, 113k 28 / 30, 135k 34 / 31, 156k
+// 36 / 40, 317k 61 / 61, 402k 75 / 69, 1.3M 224 / 195.
+constexpr EtForm kRecForm = {4, 4, 2, 1};
+
 __global__ void __launch_bounds__(kEtThreads)
 k_recovered_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
                            const double* __restrict__ y, const double* __restrict__ u, const double* __restrict__ v,
@@ -409,7 +422,7 @@ cfa_status cfa_recovered_gradient(cfa_ctx* ctx, const cfa_mesh* m, const double*
     CFA_ENTER(ctx);
     CFA_ARG(m && u && v && grad_rec && H > 0.0);
     allow_post_kernels();
-    if (m->et.ok)
+    if (et_better(m->et, m->n, ctx->num_sms, kRecForm))
         CFA_LAUNCH(ctx, k_recovered_gradient_tiles, m->et.ntiles, kEtThreads, et_smem_bytes(m->et, 5), m->tiles(), m->n, m->ev,
                    m->x, m->y, u, v, u_max, H, grad_rec);
     else

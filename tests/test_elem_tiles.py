@@ -31,6 +31,11 @@ def _wheel(spokes):
     return F.Mesh(x, y, tag, tri, np.zeros(spokes, np.int32))
 
 
+def _target(n, seed):
+    import batch as B
+    return B.batch_system(seed, n, n).mesh
+
+
 def _one():
     return F.Mesh(np.array([0.0, 1.0, 0.3]), np.array([0.0, 0.2, 0.9]), np.array([0, 2, 1], np.int32),
                   np.array([[0, 1, 2]], np.int32), np.zeros(1, np.int32))
@@ -42,6 +47,7 @@ CASES = {
     "small": lambda: F.make_mesh("small"),
     "small_shuffled": lambda: _shuffled(F.make_mesh("small")),
     "c0_rows64": lambda: F.make_mesh("c0"),
+    "37k_rows96": lambda: _target(31_001, 5),
     "medium_rows96": lambda: F.make_mesh("medium"),
     "wheel_24": lambda: _wheel(24),              # one thread plans the row
     "wheel_25": lambda: _wheel(25),              # the whole block does
@@ -169,9 +175,9 @@ def test_node_gradients_match_the_formulas(name):
 HUB = 2000   # elements around one vertex, whose records exceed a tile: the whole mesh takes the row gathers
 
 
-def _with_hub(m):
-    """`m` and, apart from it, a disc of HUB elements: m's rows as the gathers form them."""
-    w = _wheel(HUB)
+def _with_hub(m, spokes=HUB):
+    """`m` and, apart from it, a disc of elements: with HUB of them, m's rows as the gathers form them."""
+    w = _wheel(spokes)
     return F.Mesh(np.concatenate([m.x, w.x]), np.concatenate([m.y, w.y]), np.concatenate([m.tag, 0 * w.tag]).astype(np.int32),
                   np.concatenate([m.tri, w.tri + m.n]).astype(np.int32), np.concatenate([m.gen, w.gen]))
 
@@ -211,7 +217,7 @@ class _Pair:
 
 BIT_MESHES = {"one": _one, "tiny": lambda: F.make_mesh("tiny"), "small": lambda: F.make_mesh("small"),
               "small_shuffled": lambda: _shuffled(F.make_mesh("small")), "c0": lambda: F.make_mesh("c0"),
-              "medium": lambda: F.make_mesh("medium")}
+              "37k": lambda: _target(31_001, 5), "medium": lambda: F.make_mesh("medium")}
 
 
 def _empty(k):
@@ -305,3 +311,60 @@ def test_gradient_tiles_give_the_gathers_bits(name, weighted):
 
     for call in (scalar, node, stiffness, recovered):
         p.same(call)
+
+
+# ----------------------------------------------------------------------------------------------
+# which form a mesh takes
+# ----------------------------------------------------------------------------------------------
+def _sorted_by_x(m):
+    perm = np.lexsort((m.y, m.x))
+    new = np.empty_like(perm)
+    new[perm] = np.arange(m.n)
+    tri = new[m.tri]
+    e = np.argsort(tri.min(1), kind="stable")
+    return F.Mesh(m.x[perm].copy(), m.y[perm].copy(), m.tag[perm].copy(), tri[e].astype(np.int32), m.gen[e].copy())
+
+
+KERNELS = {"mom": "k_momentum", "press": "k_pressure", "grad": "k_scalar_gradient", "node": "k_node_gradients",
+           "rec": "k_recovered_gradient"}
+# kernels on tiles (148 SMs): one wave of both forms; two waves of tiles against one of gathers; the same
+# with the gathers' second wave begun; little sharing; none; none in a mesh of 64-row tiles; a hub
+ROUTES = {
+    "37k": (lambda: _target(31_001, 5), {"mom", "press", "grad", "node", "rec"}),
+    "56k": (lambda: _target(45_001, 2), {"press", "grad", "node", "rec"}),
+    "76k": (lambda: _target(60_001, 5), {"mom", "press", "node", "rec"}),
+    "37k_sorted_by_x": (lambda: _sorted_by_x(_target(31_001, 5)), {"press"}),
+    "37k_shuffled": (lambda: _shuffled(_target(31_001, 5)), set()),
+    "c0_shuffled": (lambda: _shuffled(F.make_mesh("c0")), {"mom", "press", "grad", "node", "rec"}),
+    "56k_hub": (lambda: _with_hub(_target(45_001, 2), 200), {"mom", "press", "grad", "node", "rec"}),
+}
+
+
+@pytest.mark.parametrize("name", list(ROUTES))
+def test_route(name):
+    import torch
+    import cfa_b200 as cfa
+    from oracle import oracle as O
+    from torch.profiler import ProfilerActivity, profile
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    make, tiles = ROUTES[name]
+    m = make()
+    ctx = cfa.default_context()
+    rp, ci = O.csr_build(m.n, m.elem_v)
+    dm = cfa.DeviceMesh(ctx, m, torch.from_numpy(rp).to("cuda"), torch.from_numpy(ci).to("cuda"))
+    n, nnz = dm.n, dm.nnz
+    z = lambda k: torch.ones(k, dtype=torch.float64, device="cuda")
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        cfa.assemble_momentum(ctx, dm, z(n), z(n), z(n), z(n), z(n), cfa.bdf2_params(), z(nnz), z(n), z(n), z(n))
+        cfa.assemble_ppe(ctx, dm, z(n), z(n), z(n), z(n), z(n), z(n), z(m.ne), 1e-3, 1.0, 0.3, z(nnz), z(n), z(n),
+                         apply_bc=False)
+        cfa.scalar_gradient(ctx, dm, z(n), z(m.ne), z(n), z(n))
+        cfa.grad_dp_vorticity(ctx, dm, z(n), z(n), z(n), z(n), z(n), z(n))
+        cfa.amr_indicators(ctx, dm, z(n), z(n), 1.5, 1.0, z(n), z(4 * n), z(2 * m.ne))
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events()]
+    took = {k for k, v in KERNELS.items() if any(v + "_tiles" in q for q in names)}
+    assert took == tiles
+    for k, v in KERNELS.items():
+        assert any(v in q for q in names), k
