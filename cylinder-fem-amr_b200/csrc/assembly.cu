@@ -200,8 +200,10 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
 // vertices, each with the L2 flushed first. A wave of tiles (3 x 148 of 96 rows) takes some 14 us, one of
 // gathers (2 x 148 of 256 rows) some 24, so tiles run up to 5/3 of the gathers' waves. Tiles / gathers in
 // us: 37k vertices 26 / 28, 56k 36 / 34, 76k 38 / 45, 113k 50 / 57, 135k 61 / 58, 156k 65 / 73, 317k
-// 118 / 123, 402k 144 / 149, 642k 220 / 221, 1.3M 427 / 419, 4.2M 1350 / 1317.
-constexpr EtForm kMomForm = {3, 2, 5, 3};
+// 118 / 123, 402k 144 / 149, 642k 220 / 221, 1.3M 427 / 419, 4.2M 1350 / 1317. A tile of some 260
+// elements is usual, one of 576 shares none: 402k vertices with 1% of them appended in random order
+// 204 / 159, 76k with 5% 55 / 54; a 22k mesh of 64-row tiles 24 / 36.
+constexpr EtForm kMomForm = {3, 2, 5, 3, 5 * kEtRows};
 __global__ void __launch_bounds__(kEtThreads, 3)
 k_momentum_tiles(ElemTileView tv, int n, const int* __restrict__ ev, const double* __restrict__ x,
                  const double* __restrict__ y, const int* __restrict__ tag, const int* __restrict__ rp,

@@ -61,14 +61,18 @@ inline int elem_tile_rows(int n, int num_sms) { return n < 2 * num_sms * kEtRows
 // Whether a kernel's tiles are its better form on this mesh. Both forms take whole waves of blocks, and
 // a wave of tiles costs a share of a wave of gathers that the kernel's comment states: tile_blocks and
 // row_blocks are the blocks an SM holds of each, num / den the most waves of tiles per wave of gathers.
-// A gather runs a long row in one thread (0.25 to 1.1 us an element), which tiles share.
+// A gather runs a long row in one thread (0.25 to 1.1 us an element), which tiles share. max_elems: the
+// largest tile sizes every block's shared memory, so one scattered tile (vertices appended by a
+// refinement and never renumbered) takes the L1 from all; the momentum's large records feel it.
 struct EtForm {
     int tile_blocks, row_blocks, num, den;
+    int max_elems = 1 << 30;
 };
 constexpr int kEtHubRow = 31;
 inline bool et_better(const ElemTiles& t, int n, int num_sms, const EtForm& f) {
     if (!t.ok || (t.rows == kEtRows && t.repeats > kEtRepeats)) return false;
     if (t.max_row > kEtHubRow) return true;
+    if (t.max_elems > f.max_elems) return false;
     const long long tiles = ceil_div(t.ntiles, f.tile_blocks * num_sms);
     const long long gathers = ceil_div(ceil_div(n, kThreads), f.row_blocks * num_sms);
     return tiles * f.den <= gathers * f.num;

@@ -316,13 +316,22 @@ def test_gradient_tiles_give_the_gathers_bits(name, weighted):
 # ----------------------------------------------------------------------------------------------
 # which form a mesh takes
 # ----------------------------------------------------------------------------------------------
-def _sorted_by_x(m):
-    perm = np.lexsort((m.y, m.x))
+def _renumbered(m, perm):
     new = np.empty_like(perm)
     new[perm] = np.arange(m.n)
     tri = new[m.tri]
     e = np.argsort(tri.min(1), kind="stable")
     return F.Mesh(m.x[perm].copy(), m.y[perm].copy(), m.tag[perm].copy(), tri[e].astype(np.int32), m.gen[e].copy())
+
+
+def _sorted_by_x(m):
+    return _renumbered(m, np.lexsort((m.y, m.x)))
+
+
+def _appended(m, share=0.05):
+    """A share of the vertices at the end, in random order."""
+    q = np.random.default_rng(1).permutation(m.n)[:int(share * m.n)]
+    return _renumbered(m, np.concatenate([np.setdiff1d(np.arange(m.n), q), q]))
 
 
 KERNELS = {"mom": "k_momentum", "press": "k_pressure", "grad": "k_scalar_gradient", "node": "k_node_gradients",
@@ -333,6 +342,7 @@ ROUTES = {
     "37k": (lambda: _target(31_001, 5), {"mom", "press", "grad", "node", "rec"}),
     "56k": (lambda: _target(45_001, 2), {"press", "grad", "node", "rec"}),
     "76k": (lambda: _target(60_001, 5), {"mom", "press", "node", "rec"}),
+    "76k_appended": (lambda: _appended(_target(60_001, 5)), {"press", "node", "rec"}),
     "37k_sorted_by_x": (lambda: _sorted_by_x(_target(31_001, 5)), {"press"}),
     "37k_shuffled": (lambda: _shuffled(_target(31_001, 5)), set()),
     "c0_shuffled": (lambda: _shuffled(F.make_mesh("c0")), {"mom", "press", "grad", "node", "rec"}),
