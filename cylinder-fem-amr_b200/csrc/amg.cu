@@ -152,9 +152,11 @@ __global__ void k_sg_ub(int rows, const int* __restrict__ arp, const int* __rest
 // memory (first touch 0.0 + prod, then += prod). Per entry these are the operations and their
 // order of csr_multiply's dense accumulator, whatever the batches. The columns are then written
 // sorted into the row's slice of the scratch. TABLE: entries of the largest table; a row uses the
-// power of two above twice its bound, so that probes stay short, and one that fills three quarters
-// of TABLE is left to k_sg_accum_big (cnt -1). Bound by the gathers of B's rows: all lanes fetch
-// products of several of them at once, the next batch while the current one is added. A setup at
+// power of two above twice its bound, so that probes stay short, and one of more columns than
+// T - 32 - T / 8 of the largest table (1760 of 2048) is left to k_sg_accum_big (cnt -1). Bound by
+// instruction issue where rows are many (71% of the slots on the finest level, DRAM 6%), by the gathers
+// of B's rows where they are few: all lanes fetch products of several of them at once, the next batch
+// while the current one is added. A setup at
 // 402k vertices: 8.3 ms of accumulation (a pass over the row's products for each of its columns, and
 // blocks of 1024 threads that each read every product of a long row) -> 1.5 ms.
 template <int TABLE, int WARPS>
@@ -1171,7 +1173,8 @@ static void vct(cfa_ctx* ctx, bool dry, const TiledCsr& M, int* err, const T* di
 // RING_CGU: RING_PRE of the residual r - alpha q after the CG's update, which it also does on its own
 // rows (k_cg_update's operations), with |r| and the stopping test.
 // Bound by latency at the sizes that take it (ring_rows, ring.cu): one round of gathers, then two
-// sweeps from shared memory, in place of two kernels. 8k vertices: a pair of kernels 7.4 us -> 4.1 us,
+// sweeps from shared memory, in place of two kernels. At 64k vertices a pair issues in 21% of the slots,
+// the LSU data pipe is 24% busy and 0.84 waves of blocks are in flight. 8k vertices: a pair of kernels 7.4 us -> 4.1 us,
 // the FP64 V-cycle 28.7 -> 21.0 us; 37k: 35.2 -> 31.7 us.
 enum RingOp { RING_PRE = 0, RING_JAC = 1, RING_CGU = 2 };
 
@@ -1856,7 +1859,9 @@ bool amg_prescale(const cfa_amg* amg, PreScale* out, bool fp64) {
     return true;
 }
 
-// Off unless CFA_CG_FUSE_UPDATE=1: measured on the 402k-vertex step the folded form was not
+// On ring tiles the update always rides in the pre-smoothing (k_ring, RING_CGU). In the one-sweep
+// kernels it is off unless CFA_CG_FUSE_UPDATE=1 (which also sets hierarchies up without rings):
+// measured on the 402k-vertex step the folded form was not
 // faster (13.78 against 13.60 ms without setup): the pre-smoothing pass gathers q beside r for every entry and the
 // residual pass takes the grid reduction, which cost what the update kernel's launch saved.
 static bool cg_update_fused() {

@@ -1,9 +1,10 @@
 // Atomic-free element assembly (a3-a9). A block owns a tile of consecutive rows and computes each
 // element that touches them once, into shared memory (elemtile.cuh); its threads then sum every
 // CSR entry and right-hand side entry from there, in ascending element order, and write every value
-// once, entries coalesced. Where a tile's elements do not fit (a node of very many elements), one
-// thread per matrix row gathers the contributions of the row's elements from the sorted
-// node -> element incidence, in the same order. Compared with the reference's one-thread-per-element kernels with FP64
+// once, entries coalesced. Where that is not the better form (et_better) or a tile's elements do not fit
+// (a node of very many elements), one thread per matrix row gathers the contributions of the row's
+// elements from the sorted node -> element incidence, in the same order and with the same roundings:
+// a mesh's bits do not depend on the form. Compared with the reference's one-thread-per-element kernels with FP64
 // atomicAdd into a binary-searched CSR slot (src/cfa/fem_kernels.cuh:40-282, :697-909), there
 // are no atomics and no searches, the result is deterministic, and each CSR value is written
 // exactly once (coalesced along the row).
@@ -194,8 +195,9 @@ k_momentum_rows(int n, const int* __restrict__ ev, const double* __restrict__ x,
 // Momentum rows on element tiles: the element matrix and right-hand side of every element of the
 // tile (16 doubles an element: A_ab, f_u, f_v, area / 3), then the entries, the rows and the
 // Dirichlet rows. Bound by latency: each block's chain of plan, vertices and fields, the divisions
-// and square roots of the element formula, then the entries' codes. Against the row gather: 142 ->
-// 130 us at 402k vertices (130 MB, 1.0 TB/s), 21.0 -> 13.3 us at 22.5k, 19.5 -> 13.2 us at 8k.
+// and square roots of the element formula, then the entries' codes (issue 28%, DRAM 7%, LSU 32% busy at
+// 402k vertices). Gathers -> tiles, the L2 flushed first: 149 -> 144 us at 402k vertices (77 MB of DRAM),
+// 29.7 -> 20.0 us at 22k, 27.7 -> 19.5 us at 7k.
 // Three blocks per SM (80 registers) matter: at 92 registers, two blocks, 189 against 144 us at 402k
 // vertices, each with the L2 flushed first. A wave of tiles (3 x 148 of 96 rows) takes some 14 us, one of
 // gathers (2 x 148 of 256 rows) some 24, so tiles run up to 5/3 of the gathers' waves. Tiles / gathers in
@@ -569,11 +571,12 @@ k_scalar_gradient_tiles(ElemTileView tv, int n, const int* __restrict__ ev, cons
 
 // Pressure rows on element tiles, 19 doubles an element: the symmetric K (6), grad N (6), w, 1 + s,
 // the right-hand side of each vertex (3), area / 3 and div u. The weights enter the sums by fused
-// multiply-adds, as in the row gather. Bound by shared memory: seven 8-byte reads a contribution,
-// 2.6 contributions an entry, and the records limit the blocks per SM. Staging the codes in shared
-// memory and loading offsets ahead was slower (152 us), as were blocks of 384 threads (177 us).
-// Against the row gather: 367 -> 148 us at 402k vertices (190 MB, 1.3 TB/s), 3713 -> 1650 us at 4.2M,
-// 32.2 -> 10.8 us at 22.5k, 25.1 -> 9.0 us at 8k.
+// multiply-adds, as in the row gather. Bound by latency (half of a warp's wait between instructions is
+// on global loads, DRAM 13% busy) with the LSU data pipe next (56% busy, two thirds of it the records'
+// shared-memory reads, seven a contribution and 2.6 contributions an entry); registers and records
+// leave four blocks an SM. Staging the codes in shared memory and loading offsets ahead was slower (152
+// us), as were blocks of 384 threads (177 us). Gathers -> tiles, the L2 flushed first: 373 -> 150 us at
+// 402k vertices (162 MB of DRAM, 1.1 TB/s), 3738 -> 1430 us at 4.2M, 41 -> 20.5 us at 22k, 35 -> 18.4 us at 7k.
 __global__ void __launch_bounds__(kEtThreads)
 k_pressure_tiles(ElemTileView tv, int n, int nnz, const int* __restrict__ ev, const double* __restrict__ x,
                  const double* __restrict__ y, const int* __restrict__ tag, const int* __restrict__ rp,

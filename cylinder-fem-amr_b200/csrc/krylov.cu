@@ -1561,9 +1561,9 @@ static cfa_status pcg_piece(cfa_ctx* ctx, PcgWork& W, const PcgArgs& a, int piec
             CFA_LAUNCH(ctx, k_cg_pq, gv, kThreads, 0, n, (const double*)W.pn.p, (const double*)W.q.p, st, W.part.p,
                        W.counter.p, cond);
         if (a.amg || a.prec) {
-            // the update (x, r, p, |r|, the stopping test) folded into the V-cycle's level 0 where
-            // the hierarchy allows it (opt-in), else its own kernel, which also forms the level-0
-            // pre-smoothing's scaled residual where the V-cycle takes it
+            // the update (x, r, p, |r|, the stopping test) folded into the V-cycle's level 0 on ring
+            // tiles (elsewhere only with CFA_CG_FUSE_UPDATE=1), else its own kernel, which also forms
+            // the level-0 pre-smoothing's scaled residual where the V-cycle takes it
             const bool fuse_update = !a.prec && amg_can_fuse_update(a.amg);
             PreScale ps{};
             // the direction, and where it is copied to unless it was updated in place

@@ -184,8 +184,8 @@ k_ring_fill(int n, int rows, const int* __restrict__ rp, const int* __restrict__
 }  // namespace
 
 // Rows per tile, 0 where one sweep per pass is the better form. A pair of sweeps saves a kernel
-// boundary, but its gathers go through shared memory in 3 to 4 wavefronts an entry, no fewer than
-// the one-sweep kernels' through L1, and its ring repeats work, so it pays while a sweep is mostly
+// boundary, but its gathers go through shared memory, some 21 wavefronts for a warp's 32 entries (columns,
+// values and vector), no fewer than the one-sweep kernels' through L1, and its ring repeats work, so it pays while a sweep is mostly
 // launch and latency. CG iteration with one against two sweeps per pass, best rows, FP64 / mixed:
 // 8k vertices 38.8 -> 33.2 / 36.4 -> 30.7 us, 37k 54.2 -> 51.3 / 51.6 -> 49.4 us, 69k 62.1 -> 59.8 /
 // 58.9 -> 56.8 us; 141k 89.1 -> 91.4 / 85.7 -> 85.6 us, 651k 236 -> 258 / 210 -> 218 us. The line lies
