@@ -8,7 +8,7 @@
 // sum from there, in ascending element order as the gathers do, so the sums keep their order.
 //
 // The plan is connectivity only (made with the mesh handle); coordinates and fields are read at
-// every call. It takes 43 bytes an element (65 as the buffers are sized), beside 56 of the handle's
+// every call. It takes 43 bytes an element (65 as the buffers are sized), beside 50 (75) of the handle's
 // incidences and positions; a mesh whose kernels all take the row gathers gives it back.
 #pragma once
 
