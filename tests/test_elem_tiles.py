@@ -374,6 +374,8 @@ def test_route(name):
         cfa.amr_indicators(ctx, dm, z(n), z(n), 1.5, 1.0, z(n), z(4 * n), z(2 * m.ne))
         torch.cuda.synchronize()
     names = [e.name for e in p.events()]
+    if not any("k_" in q for q in names):
+        pytest.skip("kernels cannot be recorded here")
     took = {k for k, v in KERNELS.items() if any(v + "_tiles" in q for q in names)}
     assert took == tiles
     for k, v in KERNELS.items():
